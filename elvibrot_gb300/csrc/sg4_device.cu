@@ -95,7 +95,7 @@ int desc_sizes(const evr_sg4_desc* d, DescSizes* z) {
 
 }  // namespace evr
 
-#include "sg4_items.cuh"
+#include "sg4_fixed.cuh"
 
 // The automatic launch plan's knobs (evr_sg4_set_plan): the most right-hand
 // sides per work item, and the mode-pass thread mapping (0 chosen per pass,
@@ -140,9 +140,15 @@ static const GeoKernels& geo_kernels(int geo) {
 static void launch_multi(int geo, unsigned grid, size_t smem, cudaStream_t s, const KParams* ps, int n_ctx,
                          const MItem* items, int n_items, int item_base, unsigned int* counter) {
   const GeoKernels& k = geo_kernels(geo);
+  bool fx = false;  // a launch's contexts all run in fixed point, or none does (a skipped one is blank)
+  for (int j = 0; j < n_ctx; ++j) fx = fx || ps[j].fx;
   if (n_ctx <= EVR_PB_SMALL) {
     ParamBlock<EVR_PB_SMALL> P;
     std::copy(ps, ps + n_ctx, P.p);
+    if (fx) {
+      multi_fxsmall.launch(grid, smem, s, P, items, n_items, item_base, counter);
+      return;
+    }
     bool t10 = true, grids = false;  // the kernel compiled for the contexts' operators
     for (int j = 0; j < n_ctx; ++j) {
       t10 = t10 && ps[j].type == 10 && ps[j].D <= k.fmax;
@@ -152,7 +158,7 @@ static void launch_multi(int geo, unsigned grid, size_t smem, cudaStream_t s, co
   } else {
     static thread_local ParamBlock<EVR_PB_LARGE> P;  // 17.5 KB: not on the stack
     std::copy(ps, ps + n_ctx, P.p);
-    k.large->launch(grid, smem, s, P, items, n_items, item_base, counter);
+    (fx ? &multi_fxlarge : k.large)->launch(grid, smem, s, P, items, n_items, item_base, counter);
   }
 }
 
@@ -164,15 +170,17 @@ static void launch_single(int geo, unsigned grid, size_t smem, cudaStream_t s, c
 }
 
 static int geo_ctas(int geo) { return geo_kernels(geo).ctas; }
+// ... of the kernels a launch runs (the fixed-point ones have one shape)
+static int launch_ctas(int geo, bool fx) { return fx ? EVR_FX_CTAS : geo_ctas(geo); }
 
 // Static shared memory plus the 1 KB the driver reserves per CTA, rounded up
 // to 256 bytes (queried once): the largest of a geometry's kernels, so all
-// of them keep the geometry's CTAs per SM.
-static int smem_slack(int geo) {
+// of them keep the geometry's CTAs per SM.  Index 3: the fixed-point kernels.
+static int smem_slack(int geo, bool fx) {
   static const std::vector<int> slack = [] {
-    std::vector<int> v(3, 4096);
+    std::vector<int> v(4, 4096);
+    size_t a = 0, b = 0, c = 0, d = 0;
     for (int g = 0; g < 3; ++g) {
-      size_t a = 0, b = 0, c = 0, d = 0;
       const GeoKernels& k = geo_kernels(g);
       if (k.small->static_smem(&a) != cudaSuccess || k.large->static_smem(&b) != cudaSuccess ||
           k.small10->static_smem(&c) != cudaSuccess || k.small1g->static_smem(&d) != cudaSuccess) {
@@ -181,27 +189,36 @@ static int smem_slack(int geo) {
       }
       v[g] = (int)((std::max(std::max(a, b), std::max(c, d)) + 1024 + 255) / 256 * 256);
     }
+    if (multi_fxsmall.static_smem(&a) == cudaSuccess && multi_fxlarge.static_smem(&b) == cudaSuccess)
+      v[3] = (int)((std::max(a, b) + 1024 + 255) / 256 * 256);
+    else
+      cudaGetLastError();
     return v;
   }();
-  return slack[geo];
+  return slack[fx ? 3 : geo];
 }
 
 // dynamic shared memory per CTA: the SM's 228 KB split between the resident
 // CTAs, less the slack above, so all of them fit (54.75 KB wide, 26.5 KB
-// narrow, 35.75 KB mid)
-static int geo_smem_bytes(int geo) { return (228 * 1024 / geo_ctas(geo) - smem_slack(geo)) / 256 * 256; }
+// narrow, 35.75 KB mid, 34.75 KB in fixed point)
+static int geo_smem_bytes(int geo, bool fx) {
+  return (228 * 1024 / launch_ctas(geo, fx) - smem_slack(geo, fx)) / 256 * 256;
+}
 
 // dynamic shared memory of every geometry's kernels (set at context creation)
 static cudaError_t set_smem_attributes() {
   cudaError_t e = cudaSuccess;
   for (int g = 0; g < 3 && e == cudaSuccess; ++g) {
     const GeoKernels& k = geo_kernels(g);
-    const int bytes = geo_smem_bytes(g);
+    const int bytes = geo_smem_bytes(g, false);
     e = k.small->set_smem(bytes);
     if (e == cudaSuccess) e = k.large->set_smem(bytes);
     if (e == cudaSuccess) e = k.small10->set_smem(bytes);
     if (e == cudaSuccess) e = k.small1g->set_smem(bytes);
   }
+  const int bytes = geo_smem_bytes(0, true);
+  if (e == cudaSuccess) e = multi_fxsmall.set_smem(bytes);
+  if (e == cudaSuccess) e = multi_fxlarge.set_smem(bytes);
   return e;
 }
 
@@ -299,6 +316,68 @@ __device__ void point_coords(const int* nq_of_l, const double* xcat, const int* 
   }
 }
 
+// g 2^k as a fixed-point value (|g 2^k| <= 2^58)
+__device__ __forceinline__ int2 fx_from(double g, int k) {
+  return fx_pack(__double2ll_rn(g * __hiloint2double((1023 + k) << 20, 0)));
+}
+
+// The exponent of the fixed-point metric per term (gfx_scan_kernel, one CTA a
+// term): the largest row or column sum of |G_ij| 2^(ed_i + ed_j) over its
+// points is below 2^geg.  bad: a value is not finite, or the points' own sums
+// spread by more than 2^6, which one exponent would not serve; bad[1]: G is not
+// symmetric.
+__global__ void __launch_bounds__(128) gfx_scan_kernel(const TermInfo* terms, int D, int Lp1, const double* G,
+                                                       const int* ed, int* geg, int* bad) {
+  __shared__ int hi, lo;
+  const TermInfo& T = terms[blockIdx.x];
+  int skew = 0;
+  if (threadIdx.x == 0) {
+    hi = -100000;
+    lo = 100000;
+  }
+  __syncthreads();
+  for (int q = threadIdx.x; q < T.nq; q += blockDim.x) {
+    const double* g = G + T.off_nq * D * D + q;
+    double big = 0.0;
+    bool ok = true;
+    for (int i = 0; i < D; ++i) {
+      double r = 0.0, c = 0.0;
+      for (int j = 0; j < D; ++j) {
+        const double s = exp2((double)(ed[i * Lp1 + T.l[i]] + ed[j * Lp1 + T.l[j]]));
+        const double a = g[(long long)T.nq * (D * i + j)], b = g[(long long)T.nq * (D * j + i)];
+        r += fabs(a) * s;
+        c += fabs(b) * s;
+        skew |= a != b;
+      }
+      ok = ok && r < 1e300 && c < 1e300;
+      big = fmax(big, fmax(r, c));
+    }
+    const int e = ok && big > 0.0 ? ilogb(big) + 1 : (ok ? -1000 : 1000);
+    atomicMax(&hi, e);
+    atomicMin(&lo, e);
+  }
+  if (skew) bad[1] = 1;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    geg[blockIdx.x] = hi;
+    if (hi > 150 || hi < -150 || hi - lo > 6) *bad = 1;
+  }
+}
+
+// The fixed-point metric from G, or its transpose (one CTA a term).
+__global__ void __launch_bounds__(256) gfx_convert_kernel(const TermInfo* terms, int D, int Lp1, const double* G,
+                                                          const int* ed, const int* geg, const FxTerm* fxterms,
+                                                          int2* Gfx, int transpose) {
+  const TermInfo& T = terms[blockIdx.x];
+  const long long o = T.off_nq * D * D;
+  for (int ij = 0; ij < D * D; ++ij) {
+    const int i = ij / D, j = ij - i * D;
+    const int k = ed[i * Lp1 + T.l[i]] + ed[j * Lp1 + T.l[j]] - geg[blockIdx.x] + 58;
+    for (int q = threadIdx.x; q < T.nq; q += blockDim.x)
+      Gfx[fx_g_index(D, fxterms[blockIdx.x].tile, q, transpose ? D * j + i : ij)] = fx_from(G[o + (long long)ij * T.nq + q], k);
+  }
+}
+
 // V polynomial terms as up to EVR_VFAC (mode << 8 | exponent) factors in
 // ascending mode order (-1 ends a term): the same products, in the same
 // order, as the dense exponent table, without its D loop per term.
@@ -309,7 +388,8 @@ __global__ void fields_kernel(const TermInfo* terms, long long nb_SG, const long
                               const int* nq_of_l, const double* xcat, const int* x_off, int D, int Lp1,
                               int V_nterms, const double* V_coef, const int* V_fac, double* V,
                               const double* G0, const double* G1, double* G, long long gp0, long long gp1, int nb0,
-                              long long vstride, int Gsym) {
+                              long long vstride, int Gsym, int2* Gfx, const int* geg, const int* ed, const FxTerm* fxterms, long long tile0,
+                              int Gtr) {
   for (long long gp = gp0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; gp < gp1;
        gp += (long long)gridDim.x * blockDim.x) {
     // binary search of the term owning global point gp
@@ -342,19 +422,27 @@ __global__ void fields_kernel(const TermInfo* terms, long long nb_SG, const long
         V[(long long)ab * vstride + gp - gp0] = v;
       }
     }
-    if (G) {
+    if (G || Gfx) {
       // a symmetric affine form (G0 and G1 symmetric in i, j, bit for bit)
       // gives G_ji the same FMA chain as G_ij: formed once, stored twice
       const long long nqt = T.nq;
-      double* Gt = G + (T.off_nq - gp0) * D * D + q;
+      const long long o = (T.off_nq - gp0) * D * D + q;
       for (int i = 0; i < D; ++i)
         for (int j = Gsym ? i : 0; j < D; ++j) {
           double g = G0 ? G0[i * D + j] : (i == j ? 1.0 : 0.0);
           if (G1)
             for (int k = 0; k < D; ++k) g = fma(G1[((long long)i * D + j) * D + k], Q[k], g);
           // GGiq(iq, j, i) of the term
-          Gt[nqt * ((long long)D * i + j)] = g;
-          if (Gsym) Gt[nqt * ((long long)D * j + i)] = g;
+          if (G) {
+            G[o + nqt * ((long long)D * i + j)] = g;
+            if (Gsym) G[o + nqt * ((long long)D * j + i)] = g;
+          }
+          if (Gfx) {
+            const int2 f = fx_from(g, ed[i * Lp1 + T.l[i]] + ed[j * Lp1 + T.l[j]] - geg[lo] + 58);
+            const long long t0 = fxterms[lo].tile - tile0;
+            Gfx[fx_g_index(D, t0, (int)q, Gtr ? D * j + i : D * i + j)] = f;
+            if (Gsym) Gfx[fx_g_index(D, t0, (int)q, Gtr ? D * i + j : D * j + i)] = f;
+          }
         }
     }
   }
@@ -481,6 +569,23 @@ struct evr_sg4_ctx {
   long long* d_pt_start = nullptr;    // [nb_SG] first grid point of every term
   std::vector<long long> slice_term;  // [nslices+1] term ranges
   std::vector<int> slice_item;        // [nslices+1] ranges of the sorted work list
+  // fixed-point items (sg4_fixed.cuh): the matrices and their scales, and
+  // the operator's own parts; fx: this operator runs there
+  bool fx = false;
+  bool has_G = false;                 // type 10 with a metric
+  std::vector<double> mats, x;        // host copies of d_mats and d_x
+  std::vector<int2> fxm;              // fixed-point matrices, at the same offsets
+  std::vector<FxTerm> fxterms;
+  FxTerm* d_fxterms = nullptr;
+  std::vector<int> ed;                // [D*(L+1)] exponent of d1GG's scale
+  int2* d_fxm = nullptr;
+  int* d_ed = nullptr;
+  int* d_rs = nullptr;
+  int* d_geg = nullptr;
+  int2* d_Gfx = nullptr;
+  int2* d_GfxT = nullptr;             // its transpose, for H^T (the same array when G is symmetric)
+  long long all_tiles = 0, slice_tiles = 0;  // tiles of a resident metric; those allocated (the largest slice)
+  int eK = 0;
   // host-pointer path buffers
   double* d_io = nullptr;
   size_t io_cap = 0;
@@ -521,7 +626,8 @@ static void free_ctx(evr_sg4_ctx* c) {
                   c->d_inv_idx, c->d_contrib, c->d_chunk_q, c->d_fun_chunk, c->d_part,
                   c->d_scratch, c->d_V, c->d_G, c->d_Jac, c->d_cfac,
                   c->d_sqRho, c->d_F2, c->d_F1, c->d_io, c->d_Vcoef, c->d_Vfac, c->d_G0, c->d_G1,
-                  c->d_pt_start, c->d_t1terms, c->d_t1grid};
+                  c->d_pt_start, c->d_t1terms, c->d_t1grid, c->d_fxm, c->d_fxterms, c->d_ed, c->d_rs, c->d_geg, c->d_Gfx,
+                  c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete c;
@@ -533,6 +639,95 @@ static int upload(T** dst, const T* src, size_t n) {
   CUDA_TRY(cudaMalloc((void**)dst, n * sizeof(T)));
   if (src) CUDA_TRY(cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice));
   return EVR_OK;
+}
+
+// int2 values of the 1-D matrices that a fixed-point item keeps in shared memory
+static long long fx_mats(const evr_sg4_ctx* c, const TermInfo& T) {
+  long long n = 0;
+  for (int i = 0; i < c->D; ++i) {
+    const int k = i * (c->L + 1) + T.l[i];
+    n += (long long)c->nq_of_l[k] * (2 * c->nb_of_l[k] + c->nq_of_l[k]);
+  }
+  return (n + 1) & ~1LL;
+}
+
+// (hi + lo) 2^58 in two limbs, rounded once (|lo| <= ulp(hi))
+static int2 fx_of(double hi, double lo) {
+  const double s = hi * 0x1p58, f = std::floor(s);
+  const long long y = (long long)f + std::llrint((s - f) + lo * 0x1p58);
+  const int h = (int)((y + (1 << 28)) >> 29);
+  return make_int2(h, (int)((unsigned)y - ((unsigned)h << 29)));
+}
+
+// m / norm to about twice the double's precision: the 59 bits are the matrix's own
+static int2 fx_ratio(double m, double norm) {
+  const double q = m / norm;
+  return fx_of(q, std::fma(-q, norm, m) / norm);
+}
+
+// largest absolute row sum of a row-major [rows][cols] matrix
+static double row_sum(const double* m, int rows, int cols) {
+  double big = 0.0;
+  for (int r = 0; r < rows; ++r) {
+    double s = 0.0;
+    for (int k = 0; k < cols; ++k) s += std::fabs(m[(size_t)r * cols + k]);
+    big = std::max(big, s);
+  }
+  return big;
+}
+
+// The fixed-point 1-D matrices of a context: the basis<->grid ones scaled to
+// absolute row sums of at most 2^58 by their own norms, whose product goes
+// into each term's weight, the derivatives by a power of two that serves both
+// directions (its exponent ed goes into the metric's scale).  The type-1
+// derivative matrices depend on F2 and come with the operator (fx_prepare).
+static int fx_matrices(evr_sg4_ctx* c, const std::vector<double>& weight) {
+  const int D = c->D, Lp1 = c->L + 1;
+  c->fxm.assign(c->mats.size(), make_int2(0, 0));
+  c->ed.assign((size_t)D * Lp1, 0);
+  c->fxterms.resize(c->nb_SG);
+  long long tile = 0;
+  std::vector<double> norm((size_t)D * Lp1 * 4, 1.0);  // forward B->G, G->B, transposed B->G, G->B
+  for (int k = 0; k < D * Lp1; ++k) {
+    const int nb = c->nb_of_l[k], nq = c->nq_of_l[k];
+    for (int t = 0; t < 2; ++t)
+      for (int w = 0; w < 2; ++w) {
+        const int o = c->mat_off[k * 8 + 4 * t + (w ? M_GB : M_BG)];
+        const double n = w ? row_sum(&c->mats[o], nb, nq) : row_sum(&c->mats[o], nq, nb);
+        if (!(n > 1e-30 && n < 1e30)) return 0;  // the FP64 items keep such a basis
+        norm[(size_t)k * 4 + 2 * t + w] = n;
+        for (int e = 0; e < nb * nq; ++e) c->fxm[o + e] = fx_ratio(c->mats[o + e], n);
+      }
+    const double n = std::max(row_sum(&c->mats[c->mat_off[k * 8 + M_D1]], nq, nq),
+                              row_sum(&c->mats[c->mat_off[k * 8 + 4 + M_D1]], nq, nq));
+    if (!(n < 1e30)) return 0;
+    const int ed = n > 1e-30 ? std::ilogb(n) + 1 : 0;
+    c->ed[k] = ed;
+    for (int t = 0; t < 2; ++t) {
+      const int o = c->mat_off[k * 8 + 4 * t + M_D1];
+      for (int e = 0; e < nq * nq; ++e) c->fxm[o + e] = fx_of(std::ldexp(c->mats[o + e], -ed), 0.0);
+    }
+  }
+  for (long long t = 0; t < c->nb_SG; ++t) {
+    if (fx_mats(c, c->terms[t]) > 4096) return 0;  // they stay in shared memory beside the work arrays
+    // the products as double-double (Dekker): one rounding at the end
+    for (int d = 0; d < 2; ++d) {
+      double hi = weight[t], lo = 0.0;
+      for (int i = 0; i < D; ++i)
+        for (int w = 0; w < 2; ++w) {
+          const double n = norm[(size_t)(i * Lp1 + c->terms[t].l[i]) * 4 + 2 * d + w];
+          const double p = hi * n;
+          lo = std::fma(hi, n, -p) + lo * n;
+          hi = p;
+        }
+      if (!(std::fabs(hi + lo) < 1e200)) return 0;
+      c->fxterms[t].wf[d] = hi + lo;
+    }
+    c->fxterms[t].tile = tile;
+    tile += (c->terms[t].nq + FX_TILE - 1) / FX_TILE;
+  }
+  c->all_tiles = tile;
+  return 1;
 }
 
 extern "C" const char* evr_sg4_last_error(void) { return g_err.c_str(); }
@@ -567,8 +762,9 @@ extern "C" int evr_sg4_create(const evr_sg4_desc* d, evr_sg4_ctx** out) {
   cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device);
   c->nb_of_l.assign(d->nb_of_l, d->nb_of_l + D * Lp1);
   c->nq_of_l.assign(d->nq_of_l, d->nq_of_l + D * Lp1);
+  c->x.assign(d->x, d->x + std::accumulate(c->nq_of_l.begin(), c->nq_of_l.end(), (size_t)0));
   // matrices, re-laid out row-major [nout][nin]
-  std::vector<double> mats;
+  std::vector<double>& mats = c->mats;
   c->mat_off.resize((size_t)D * Lp1 * 8);
   c->x_off.resize((size_t)D * Lp1);
   size_t o_rgb = 0, o_gb = 0, o_gg = 0, o_x = 0;
@@ -687,7 +883,8 @@ extern "C" int evr_sg4_create(const evr_sg4_desc* d, evr_sg4_ctx** out) {
   // launch geometry: persistent CTAs per SM sharing ~220 KB of shared memory
   // (wide until a work plan chooses otherwise)
   c->geo = 0;
-  c->smem_doubles = geo_smem_bytes(0) / 8;
+  if (D > FX_MAXD || !fx_matrices(c, std::vector<double>(d->weight, d->weight + d->nb_SG))) c->fxm.clear();
+  c->smem_doubles = geo_smem_bytes(0, false) / 8;
   c->grid = geo_ctas(0) * c->num_sms;
   if ((rc = upload(&c->d_map, d->map, (size_t)z.sum_nb)) ||
       (rc = upload(&c->d_mats, mats.data(), mats.size())) ||
@@ -703,6 +900,12 @@ extern "C" int evr_sg4_create(const evr_sg4_desc* d, evr_sg4_ctx** out) {
       (rc = upload(&c->d_inv_idx, inv_idx.data(), inv_idx.size())) ||
       (rc = upload(&c->d_chunk_q, chunk_q.data(), chunk_q.size())) ||
       (rc = upload(&c->d_fun_chunk, fun_chunk.data(), fun_chunk.size()))) {
+    free_ctx(c);
+    return rc;
+  }
+  if (!c->fxm.empty() && ((rc = upload(&c->d_fxm, c->fxm.data(), c->fxm.size())) ||
+                          (rc = upload(&c->d_ed, c->ed.data(), c->ed.size())) ||
+                          (rc = upload(&c->d_fxterms, c->fxterms.data(), c->fxterms.size())))) {
     free_ctx(c);
     return rc;
   }
@@ -724,13 +927,17 @@ extern "C" int evr_sg4_destroy(evr_sg4_ctx* c) {
 
 // V (polynomial) and/or G (affine) on the grid points [g0, g1) (whole terms) into
 // the context's field arrays, from index 0.
-static int eval_fields(evr_sg4_ctx* c, long long g0, long long g1, bool V, bool G, cudaStream_t s) {
+// transpose: the fixed-point metric of a streamed slice for H^T.
+static int eval_fields(evr_sg4_ctx* c, long long g0, long long g1, bool V, bool G, cudaStream_t s, long long tile0 = 0,
+                       bool transpose = false) {
   if (g1 <= g0) return EVR_OK;
   const long long blocks = std::max<long long>(1, std::min<long long>((g1 - g0 + 255) / 256, 8LL * c->num_sms));
   fields_kernel<<<(unsigned)blocks, 256, 0, s>>>(c->d_terms, c->nb_SG, c->d_pt_start, c->d_nq_of_l, c->d_x,
                                                  c->d_x_off, c->D, c->L + 1, V ? c->V_nterms : 0, c->d_Vcoef,
                                                  c->d_Vfac, V ? c->d_V : nullptr, c->d_G0, c->d_G1,
-                                                 G ? c->d_G : nullptr, g0, g1, c->nb0, c->z.sum_nq, c->G_sym);
+                                                 G ? c->d_G : nullptr, g0, g1, c->nb0, c->z.sum_nq, c->G_sym,
+                                                 G ? c->d_Gfx : nullptr, c->d_geg, c->d_ed, c->d_fxterms, tile0,
+                                                 transpose);
   CUDA_TRY(cudaGetLastError());
   return EVR_OK;
 }
@@ -748,6 +955,142 @@ extern "C" int evr_sg4_field_slices(const evr_sg4_ctx* c, long long* nslices) {
   return EVR_OK;
 }
 
+// Whether this operator runs in fixed point, decided from the call's host data
+// (before any field is evaluated, so that resident and streamed fields of one
+// operator agree), with the type-1 derivative matrices and the exponents of an
+// affine metric.  Fixed point takes one channel, D <= FX_MAXD, types 0, 1 with
+// constant diagonal F2, and 10 with a metric and no volume factors, and fields
+// within 2^+-150; one exponent per term has to serve its metric, so an affine
+// metric may exceed its constant part by at most 2^6 (a metric grid is checked
+// on the device).  The other operators keep the FP64 items.
+static bool fx_prepare(evr_sg4_ctx* c, const evr_sg4_op_desc* op, bool polyV, bool affG, std::vector<int>& geg) {
+  const int D = c->D, Lp1 = c->L + 1;
+  if (c->fxm.empty() || c->nb0 > 1) return false;
+  auto inside = [](double v) { return v == 0.0 || (v > 0x1p-150 && v < 0x1p150); };
+  std::vector<double> qmax((size_t)D * Lp1, 0.0), qall(D, 0.0);  // largest |Q| per (mode, level), per mode
+  for (int k = 0; k < D * Lp1; ++k) {
+    for (int q = 0; q < c->nq_of_l[k]; ++q) qmax[k] = std::max(qmax[k], std::fabs(c->x[c->x_off[k] + q]));
+    qall[k / Lp1] = std::max(qall[k / Lp1], qmax[k]);
+  }
+  double vmax = 0.0;
+  if (op->V_grid)
+    for (long long k = 0; k < c->z.sum_nq; ++k) vmax = std::max(vmax, std::fabs(op->V_grid[k]));
+  else if (polyV)
+    for (int t = 0; t < op->V_nterms; ++t) {
+      double m = std::fabs(op->V_coef[t]);
+      for (int i = 0; i < D; ++i) m *= std::pow(qall[i], op->V_expo[t * D + i]);
+      vmax += m;
+    }
+  if (!inside(vmax)) return false;
+  if (op->type == 1) {
+    if (op->F2_grid || op->F1_grid || t1_mixed(c)) return false;
+    std::vector<double> n((size_t)D * Lp1, 0.0);
+    double sum = 0.0;
+    for (int i = 0; i < D; ++i) {
+      double big = 0.0;
+      for (int l = 0; l < Lp1; ++l) {
+        const int k = i * Lp1 + l, nq = c->nq_of_l[k];
+        n[k] = std::fabs(c->F2[i * D + i]) * std::max(row_sum(&c->mats[c->mat_off[k * 8 + M_D2]], nq, nq),
+                                                      row_sum(&c->mats[c->mat_off[k * 8 + 4 + M_D2]], nq, nq));
+        big = std::max(big, n[k]);
+      }
+      sum += big;
+    }
+    if (!inside(sum)) return false;
+    c->eK = sum > 0.0 ? std::ilogb(sum) + 1 : 0;
+    std::vector<int> rs((size_t)D * Lp1, 0);
+    for (int k = 0; k < D * Lp1; ++k) {
+      const double f = c->F2[(k / Lp1) * (D + 1)];
+      if (f == 0.0) continue;
+      rs[k] = (int)std::ceil(std::ldexp(n[k], 30 - c->eK)) + 1;
+      for (int t = 0; t < 2; ++t) {
+        const int o = c->mat_off[k * 8 + 4 * t + M_D2], nq = c->nq_of_l[k];
+        for (int e = 0; e < nq * nq; ++e) {
+          const double m = f * c->mats[o + e];
+          c->fxm[o + e] = fx_of(std::ldexp(m, -c->eK), std::ldexp(std::fma(f, c->mats[o + e], -m), -c->eK));
+        }
+      }
+    }
+    if (cudaMemcpy(c->d_fxm, c->fxm.data(), c->fxm.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess ||
+        upload(&c->d_rs, rs.data(), rs.size())) {
+      cudaGetLastError();
+      return false;
+    }
+  } else if (op->type == 10) {
+    if (op->Jac_grid || op->sqRho_grid || (!op->G_grid && !affG)) return false;
+    if (affG) {
+      geg.resize(c->nb_SG);
+      std::vector<double> g0(D * D), g1(D * D * D, 0.0), g(D * D), s(D);  // |G0|, |G1|, their bound on the term
+      for (int e = 0; e < D * D; ++e) g0[e] = op->G0 ? std::fabs(op->G0[e]) : (e % (D + 1) == 0 ? 1.0 : 0.0);
+      for (int e = 0; op->G1 && e < D * D; ++e)
+        for (int k = 0; k < D; ++k) g1[(size_t)k * D * D + e] = std::fabs(op->G1[(size_t)e * D + k]);
+      for (long long t = 0; t < c->nb_SG; ++t) {
+        const unsigned char* l = c->terms[t].l;
+        g = g0;
+        for (int k = 0; k < D; ++k) {
+          const double q = qmax[k * Lp1 + l[k]];
+          for (int e = 0; e < D * D; ++e) g[e] += g1[(size_t)k * D * D + e] * q;
+          s[k] = std::ldexp(1.0, c->ed[k * Lp1 + l[k]]);
+        }
+        double big = 0.0, big0 = 0.0;
+        for (int i = 0; i < D; ++i) {
+          double r = 0.0, q = 0.0, r0 = 0.0;
+          for (int j = 0; j < D; ++j) {
+            r += g[i * D + j] * s[j];
+            q += g[j * D + i] * s[j];
+            r0 += g0[i * D + j] * s[j];
+          }
+          big = std::max(big, std::max(r, q) * s[i]);
+          big0 = std::max(big0, r0 * s[i]);
+        }
+        if (!(big > 0x1p-150 && big < 0x1p150 && big <= 64.0 * big0)) return false;
+        geg[t] = std::ilogb(big) + 1;
+      }
+    }
+  }
+  return true;
+}
+
+// The fixed-point grid of a resident metric G (c->d_G on the device; affine:
+// evaluated into d_Gfx with the double one), and its transpose if G is not
+// symmetric.  Without memory for them, or with a metric that one exponent per
+// term does not serve, the operator stays with the FP64 items.
+static int fx_metric(evr_sg4_ctx* c, bool affine) {
+  const int D = c->D;
+  const size_t bytes = (size_t)c->slice_tiles * fx_tile_size(D) * sizeof(int2);
+  int flags[2] = {0, affine && !c->G_sym};
+  if (!affine) {
+    int* d_flags = nullptr;
+    CUDA_TRY(cudaMemcpy(c->d_terms, c->terms.data(), c->terms.size() * sizeof(TermInfo), cudaMemcpyHostToDevice));
+    int rc = upload(&d_flags, flags, 2);
+    if (!rc) rc = upload<int>(&c->d_geg, nullptr, c->terms.size());
+    if (!rc) {
+      gfx_scan_kernel<<<(unsigned)c->nb_SG, 128>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg, d_flags);
+      if (cudaMemcpy(flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost) != cudaSuccess)
+        rc = set_error(EVR_ERR_CUDA, "set_operator: metric scan: %s", cudaGetErrorString(cudaGetLastError()));
+    }
+    if (d_flags) cudaFree(d_flags);
+    if (rc) return rc;
+  }
+  if (flags[0] || (!affine && cudaMalloc(&c->d_Gfx, bytes) != cudaSuccess) ||
+      (flags[1] && cudaMalloc(&c->d_GfxT, bytes) != cudaSuccess)) {
+    cudaGetLastError();
+    if (c->d_Gfx) cudaFree(c->d_Gfx);
+    c->d_Gfx = c->d_GfxT = nullptr;
+    c->fx = false;
+    return EVR_OK;
+  }
+  if (!affine)
+    gfx_convert_kernel<<<(unsigned)c->nb_SG, 256>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg,
+                                                  c->d_fxterms, c->d_Gfx, 0);
+  if (flags[1])
+    gfx_convert_kernel<<<(unsigned)c->nb_SG, 256>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg,
+                                                  c->d_fxterms, c->d_GfxT, 1);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaDeviceSynchronize());
+  return EVR_OK;
+}
+
 extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
   if (!c || !op) return set_error(EVR_ERR_ARG, "evr_sg4_set_operator: NULL argument");
   if (op->type != 0 && op->type != 1 && op->type != 10)
@@ -760,6 +1103,12 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       cudaFree(*p);
       *p = nullptr;
     }
+  void* fxp[] = {c->d_rs, c->d_geg, c->d_Gfx, c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT};
+  for (void* q : fxp)
+    if (q) cudaFree(q);
+  c->d_rs = c->d_geg = nullptr;
+  c->d_Gfx = c->d_GfxT = nullptr;
+  c->fx = c->has_G = false;
   if (c->d_t1terms) cudaFree(c->d_t1terms);
   c->d_t1terms = nullptr;
   c->n_t1 = 0;
@@ -800,12 +1149,12 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
   const bool stream = c->field_budget > 0 && !grids && (polyV || affG) && bpp * (double)snq > (double)c->field_budget;
   if (stream && c->nb0 > 1)
     return set_error(EVR_ERR_ARG, "field budget: streamed fields take one channel (nb0 = %d)", c->nb0);
-  long long slice_pts = snq;
+  long long slice_pts = snq, slice_tiles = c->all_tiles;
   if (stream) {
     const long long cap = (long long)((double)c->field_budget / bpp);
     c->slice_term.push_back(0);
-    long long pts = 0;
-    slice_pts = 0;
+    long long pts = 0, tiles = 0;
+    slice_pts = slice_tiles = 0;
     for (long long t = 0; t < c->nb_SG; ++t) {
       const long long q = c->terms[t].nq;
       if (q > cap)
@@ -813,10 +1162,12 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
                          c->field_budget, t, q);
       if (pts + q > cap) {
         c->slice_term.push_back(t);
-        pts = 0;
+        pts = tiles = 0;
       }
       pts += q;
+      tiles += (q + FX_TILE - 1) / FX_TILE;
       slice_pts = std::max(slice_pts, pts);
+      slice_tiles = std::max(slice_tiles, tiles);
     }
     c->slice_term.push_back(c->nb_SG);
   }
@@ -825,12 +1176,32 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       if (!std::isfinite(op->V_grid[k])) return set_error(EVR_ERR_NUMERIC, "V_grid[%lld] is not finite", k);
     if ((rc = upload(&c->d_V, op->V_grid, (size_t)nvg))) return rc;
   }
+  memset(c->F2, 0, sizeof(c->F2));
+  memset(c->F1, 0, sizeof(c->F1));
+  if (op->type == 1) {
+    if (op->F2)
+      for (int i = 0; i < D; ++i)
+        for (int j = i; j < D; ++j) c->F2[i * D + j] = op->F2[i * D + j];
+    if (op->F1)
+      for (int i = 0; i < D; ++i) c->F1[i] = op->F1[i];
+  }
+  std::vector<int> geg;
+  c->has_G = op->type == 10 && (op->G_grid || affG);
+  bool fx = fx_prepare(c, op, polyV, affG, geg);
   if (polyV) CUDA_TRY(cudaMalloc(&c->d_V, (size_t)slice_pts * 8 * c->nb0 * c->nb0));
   if (op->type == 10) {
     if (op->G_grid) {
       if ((rc = upload(&c->d_G, op->G_grid, (size_t)snq * D * D))) return rc;
     } else if (affG) {
-      CUDA_TRY(cudaMalloc(&c->d_G, (size_t)slice_pts * D * D * 8));
+      // streamed: the metric in the form that the items read; resident: in both
+      if (!fx || !stream) CUDA_TRY(cudaMalloc(&c->d_G, (size_t)slice_pts * D * D * 8));
+      if (fx && cudaMalloc(&c->d_Gfx, (size_t)slice_tiles * fx_tile_size(D) * sizeof(int2)) != cudaSuccess) {
+        cudaGetLastError();
+        c->d_Gfx = nullptr;
+        if (stream) return set_error(EVR_ERR_ALLOC, "set_operator: no memory for a slice of the metric");
+        fx = false;
+      }
+      if (fx && (rc = upload(&c->d_geg, geg.data(), geg.size()))) return rc;
     }
     if (op->Jac_grid) {
       for (long long k = 0; k < snq; ++k)
@@ -850,15 +1221,6 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
         cf[k] = -0.5 / ((op->Jac_grid ? op->Jac_grid[k] : 1.0) * (op->sqRho_grid ? op->sqRho_grid[k] : 1.0));
       if ((rc = upload(&c->d_cfac, cf.data(), cf.size()))) return rc;
     }
-  }
-  memset(c->F2, 0, sizeof(c->F2));
-  memset(c->F1, 0, sizeof(c->F1));
-  if (op->type == 1) {
-    if (op->F2)
-      for (int i = 0; i < D; ++i)
-        for (int j = i; j < D; ++j) c->F2[i * D + j] = op->F2[i * D + j];
-    if (op->F1)
-      for (int i = 0; i < D; ++i) c->F1[i] = op->F1[i];
   }
   if (op->type == 1 && (op->F2_grid || op->F1_grid)) {
     // Q-dependent coefficients: the term list in Init_TypeOp order, (i, j >= i)
@@ -938,6 +1300,10 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       CUDA_TRY(cudaDeviceSynchronize());
     }
   }
+  c->fx = fx;
+  c->slice_tiles = slice_tiles;
+  if (fx && op->type == 10 && !stream && (rc = fx_metric(c, op->G_grid == nullptr))) return rc;
+  if (c->fx && !c->d_GfxT) c->d_GfxT = c->d_Gfx;  // streamed: the slice is evaluated for the direction asked for
   c->streamed = stream;
   c->have_op = true;
   return EVR_OK;
@@ -945,34 +1311,50 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
 
 
 // Work list of one H.psi over nrhs_v virtual right-hand sides: (term, rhs
-// block) items in term order with their costs, and the term table with each
-// term's block size r for this nrhs_v (the context itself is not modified).
-static void plan_work(const evr_sg4_ctx* c, int nrhs_v, int smem_doubles, std::vector<TermInfo>& terms,
-                      std::vector<Item>& items, std::vector<float>& cost, long long& max_need) {
-  const int nbuf = nbuf_for(c);
-  const int Rmax = c->rmax;
-  max_need = 0;
+// block) items in term order with their costs, the term table with each
+// term's block size r for this nrhs_v, and the doubles of global scratch that
+// a CTA needs (the context itself is not modified).  Fixed-point items (fx)
+// take one column or a pair, which shares every matrix and metric load; of the
+// work arrays, those that do not fit in shared memory go to the scratch slab.
+static void plan_work(const evr_sg4_ctx* c, bool fx, int nrhs_v, int smem_doubles, int rcap,
+                      std::vector<TermInfo>& terms, std::vector<Item>& items, std::vector<float>& cost,
+                      long long& slab) {
+  const int nbuf = fx ? (c->type == 10 ? c->D + 1 : 2) : nbuf_for(c);
+  slab = 0;
   items.clear();
   cost.clear();
   if (&terms != &c->terms) terms = c->terms;
   for (long long t = 0; t < c->nb_SG; ++t) {
     TermInfo& T = terms[t];
-    long long per = (long long)nbuf * T.nq;
-    int r = (int)std::min<long long>(std::min(nrhs_v, Rmax), std::max<long long>(1, smem_doubles / per));
-    if (c->nb0 > 1) {  // whole channel groups (both halves of complex columns): 2 nb0 columns
-      const int g = 2 * c->nb0;
-      r = std::max(g, r / g * g);
+    const long long per = (long long)nbuf * T.nq;
+    int r;
+    if (fx) {
+      const long long room = smem_doubles - fx_mats(c, T);
+      const int want = std::min(nrhs_v, rcap);
+      r = std::min(want, (int)FX_MAXR);
+      const long long fit = std::min<long long>(nbuf, room / ((long long)T.nq * r));
+      slab = std::max(slab, (nbuf - fit) * T.nq * r);
+      if (per > smem_doubles) slab = std::max(slab, per);  // a column left to the FP64 code
+    } else {
+      r = (int)std::min<long long>(std::min(nrhs_v, rcap), std::max<long long>(1, smem_doubles / per));
+      if (c->nb0 > 1) {  // whole channel groups (both halves of complex columns): 2 nb0 columns
+        const int g = 2 * c->nb0;
+        r = std::max(g, r / g * g);
+      }
+      if (per * r > smem_doubles) slab = std::max(slab, per * r);
     }
     T.r = r;
-    max_need = std::max(max_need, per * r);
     double fl = 0;  // cost ~ grid size times the 1-D lengths
     for (int i = 0; i < c->D; ++i) fl += c->nq_of_l[i * (c->L + 1) + T.l[i]];
     T.cost = (float)(fl * T.nq);
-    for (int r0 = 0; r0 < nrhs_v; r0 += r) {
-      items.push_back(Item{(int)t, r0});
-      cost.push_back(T.cost * std::min(r, nrhs_v - r0));
+    for (int r0 = 0; r0 < nrhs_v;) {
+      int n = std::min(r, nrhs_v - r0);
+      items.push_back(Item{(int)t, r0, n});
+      cost.push_back(T.cost * n);
+      r0 += n;
     }
   }
+  slab = (slab + 1) & ~1LL;  // pairs of columns are loaded as 16 bytes
 }
 
 // Geometry of a plan with n_wide items planned for the wide kernel: plans of
@@ -986,11 +1368,12 @@ static int choose_geo(int D, size_t n_wide, int num_sms) {
 // balanced), with each term's block size written into `terms`, and the
 // launch geometry chosen for this plan (the context is not modified).
 static void plan_sorted(const evr_sg4_ctx* c, int nrhs_v, std::vector<TermInfo>& terms, std::vector<Item>& items,
-                        std::vector<Item>& sorted, long long& max_need, int& geo) {
+                        std::vector<Item>& sorted, long long& slab, int& geo, int rcap = 1 << 30) {
   std::vector<float> cost;
-  plan_work(c, nrhs_v, geo_smem_bytes(0) / 8, terms, items, cost, max_need);
+  rcap = std::min(rcap, c->rmax);
+  plan_work(c, c->fx, nrhs_v, geo_smem_bytes(0, c->fx) / 8, rcap, terms, items, cost, slab);
   geo = c->geo_override >= 0 ? c->geo_override : choose_geo(c->D, items.size(), c->num_sms);
-  if (geo) plan_work(c, nrhs_v, geo_smem_bytes(geo) / 8, terms, items, cost, max_need);
+  if (geo) plan_work(c, c->fx, nrhs_v, geo_smem_bytes(geo, c->fx) / 8, rcap, terms, items, cost, slab);
   std::vector<int> order(items.size());
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
@@ -1001,26 +1384,26 @@ static void plan_sorted(const evr_sg4_ctx* c, int nrhs_v, std::vector<TermInfo>&
 // plan_sorted into the context's own term table and launch geometry
 // (c->terms, c->geo, c->smem_doubles, c->grid).
 static void plan_items(evr_sg4_ctx* c, int nrhs_v, std::vector<Item>& items, std::vector<Item>& sorted,
-                       long long& max_need) {
+                       long long& slab) {
   int geo = 0;
-  plan_sorted(c, nrhs_v, c->terms, items, sorted, max_need, geo);
+  plan_sorted(c, nrhs_v, c->terms, items, sorted, slab, geo);
   c->geo = geo;
-  c->smem_doubles = geo_smem_bytes(geo) / 8;
-  c->grid = geo_ctas(geo) * c->num_sms;
+  c->smem_doubles = geo_smem_bytes(geo, c->fx) / 8;
+  c->grid = launch_ctas(geo, c->fx) * c->num_sms;
 }
 
 // a single context's device work list: every item in slot 0
 static std::vector<MItem> slot0_items(const std::vector<Item>& items) {
   std::vector<MItem> out(items.size());
-  for (size_t k = 0; k < items.size(); ++k) out[k] = MItem{0, items[k].term, items[k].rhs0, 0};
+  for (size_t k = 0; k < items.size(); ++k) out[k] = MItem{0, items[k].term, items[k].rhs0, items[k].r};
   return out;
 }
 
 static int build_items(evr_sg4_ctx* c, int nrhs_v) {
   if (c->items_nrhs == nrhs_v) return EVR_OK;
   std::vector<Item> items, sorted;
-  long long max_need = 0;
-  plan_items(c, nrhs_v, items, sorted, max_need);
+  long long per_cta = 0;
+  plan_items(c, nrhs_v, items, sorted, per_cta);
   // streamed fields: the list runs slice by slice (decreasing cost within a slice)
   c->slice_item.assign(1, 0);
   if (c->streamed) {
@@ -1063,7 +1446,6 @@ static int build_items(evr_sg4_ctx* c, int nrhs_v) {
   CUDA_TRY(cudaMemcpy(c->d_terms, c->terms.data(), c->terms.size() * sizeof(TermInfo), cudaMemcpyHostToDevice));
   c->n_items = (int)items.size();
   // global scratch for terms that do not fit in shared memory
-  long long per_cta = max_need > c->smem_doubles ? max_need : 0;
   if ((size_t)per_cta * c->grid > c->scratch_cap) {
     if (c->d_scratch) cudaFree(c->d_scratch);
     c->d_scratch = nullptr;
@@ -1147,7 +1529,21 @@ static KParams make_params(evr_sg4_ctx* c, int nrhs_v, int cshift, const double*
   p.nb0 = c->nb0;
   p.Nfun = c->N;
   p.vstride = c->z.sum_nq;
+  p.fx = c->fx ? 1 : 0;
+  p.fxm = c->d_fxm;
+  p.fxterms = c->d_fxterms;
+  p.Gfx = c->d_Gfx;  // use_transpose swaps it
+  p.geg = c->d_geg;
+  p.ed = c->d_ed;
+  p.rs = c->d_rs;
+  p.eK = c->eK;
   return p;
+}
+
+// H^T: the transposed matrices (chosen in the items) and metric.
+static void use_transpose(KParams& p, const evr_sg4_ctx* c, int transpose) {
+  p.transpose = transpose ? 1 : 0;
+  p.Gfx = transpose ? c->d_GfxT : c->d_Gfx;
 }
 
 static int hpsi_common(evr_sg4_ctx* c, int nrhs, int cshift, const double* psi, long long ldpsi,
@@ -1175,17 +1571,19 @@ static int hpsi_common(evr_sg4_ctx* c, int nrhs, int cshift, const double* psi, 
   cudaStream_t s = (cudaStream_t)stream;
   const long long ldv_psi = ldpsi << cshift, ldv_h = ldh << cshift;
   KParams p = make_params(c, nrhs_v, cshift, psi, ldv_psi, hpsi, ldv_h, 1.0);
-  p.transpose = transpose ? 1 : 0;
+  use_transpose(p, c, transpose);
   const size_t smem = (size_t)c->smem_doubles * 8;
   long long launches = 0;
   if (!plain && c->streamed) {  // per slice: its fields, then its items
     for (size_t k = 0; k + 1 < c->slice_term.size(); ++k) {
       const long long t0 = c->slice_term[k], t1 = c->slice_term[k + 1];
       const long long g0 = c->terms[t0].off_nq, g1 = t1 < c->nb_SG ? c->terms[t1].off_nq : c->z.sum_nq;
-      if ((rc = eval_fields(c, g0, g1, c->V_nterms > 0, c->d_G1 || c->d_G0, s))) return rc;
+      const long long tile0 = c->fxterms.empty() ? 0 : c->fxterms[t0].tile;
+      if ((rc = eval_fields(c, g0, g1, c->V_nterms > 0, c->d_G1 || c->d_G0, s, tile0, transpose))) return rc;
       CUDA_TRY(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned int), s));
       KParams q = p;
       q.fbase = g0;
+      q.tbase = tile0;
       launch_single(c->geo, c->grid, smem, s, q, c->d_items + c->slice_item[k],
                     c->slice_item[k + 1] - c->slice_item[k], c->d_counter);
       CUDA_TRY(cudaGetLastError());
@@ -1320,7 +1718,7 @@ extern "C" int evr_sg4_flops_per_rhs(const evr_sg4_ctx* c, double* flops) {
       }
     } else {
       f += 4.0 * q * sum_nqi;                       // D derivative passes, twice
-      f += c->d_G ? 2.0 * D * D * q : 0.0;           // G contraction
+      f += c->has_G ? 2.0 * D * D * q : 0.0;         // G contraction
       f += (c->d_Jac ? 2.0 * D * q : 0.0) + (c->d_sqRho ? 2.0 * q : 0.0);
       f += vq + 2.0 * q;                            // V.x and the final multiply-add
     }
@@ -1496,23 +1894,32 @@ extern "C" int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi,
   // this call's plan, in local copies: the context's cached plan stays as it is
   std::vector<TermInfo> terms;
   std::vector<Item> items, sorted;
-  long long max_need = 0;
+  long long per_cta = 0;
   int geo = 0;
-  plan_sorted(c, nrhs_v, terms, items, sorted, max_need, geo);
-  const int smem_doubles = geo_smem_bytes(geo) / 8;
+  plan_sorted(c, nrhs_v, terms, items, sorted, per_cta, geo);
+  int smem_doubles = geo_smem_bytes(geo, c->fx) / 8;
   // carve: [counter | terms | items | contributions | chunk partials | large-term slabs], 256-byte aligned
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-  const size_t off_terms = 256;
-  const size_t off_items = off_terms + up(terms.size() * sizeof(TermInfo));
-  const size_t off_contrib = off_items + up(sorted.size() * sizeof(MItem));
-  const size_t off_part = off_contrib + up((size_t)c->z.sum_nb * nrhs_v * 8);
-  const size_t off_slabs = off_part + up((size_t)c->n_chunks * nrhs_v * 16);
-  const long long per_cta = max_need > smem_doubles ? max_need : 0;
-  // with large-term slabs, launch only as many CTAs as the array has slabs for
-  int grid = geo_ctas(geo) * c->num_sms;
-  if (per_cta > 0 && off_slabs < (size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES)
-    grid = (int)std::min<long long>(grid, ((size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES - off_slabs) / ((size_t)per_cta * 8));
-  const size_t total = off_slabs + (size_t)per_cta * std::max(grid, 1) * 8;
+  size_t off_terms, off_items, off_contrib, off_part, off_slabs, total;
+  int grid;
+  auto carve = [&]() {
+    off_terms = 256;
+    off_items = off_terms + up(terms.size() * sizeof(TermInfo));
+    off_contrib = off_items + up(sorted.size() * sizeof(MItem));
+    off_part = off_contrib + up((size_t)c->z.sum_nb * nrhs_v * 8);
+    off_slabs = off_part + up((size_t)c->n_chunks * nrhs_v * 16);
+    // with large-term slabs, launch only as many CTAs as the array has slabs for
+    grid = launch_ctas(geo, c->fx) * c->num_sms;
+    if (per_cta > 0 && off_slabs < (size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES)
+      grid = (int)std::min<long long>(grid, ((size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES - off_slabs) / ((size_t)per_cta * 8));
+    total = off_slabs + (size_t)per_cta * std::max(grid, 1) * 8;
+  };
+  carve();
+  if (c->fx && (grid < 1 || total > (size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES)) {  // one column an item takes the least
+    plan_sorted(c, nrhs_v, terms, items, sorted, per_cta, geo, 1);
+    smem_doubles = geo_smem_bytes(geo, true) / 8;
+    carve();
+  }
   if (grid < 1 || total > (size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES)
     return set_error(EVR_ERR_ARG,
                      "hpsi_noalloc: this operator and nrhs=%d need %zu bytes of scratch, more than the fixed "
@@ -1565,6 +1972,7 @@ struct evr_sg4_multi {
   int n = 0, cshift = 0, transpose = 0;
   std::vector<evr_sg4_ctx*> ctxs;
   std::vector<int> nrhs_v, type, nbuf;  // per context; type and work arrays per point fix the plan
+  std::vector<char> fx;          // per context: in fixed point (whole launch groups are, or are not)
   std::vector<int> group;        // per context: its launch group
   std::vector<int> slot;         // per context: its slot in that group's parameter block
   std::vector<MGroup> groups;    // one, or two when D <= 6 contexts fill a narrow launch of their own;
@@ -1598,8 +2006,9 @@ static void free_multi(evr_sg4_multi* m) {
   delete m;
 }
 
-extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int flags,
-                                    evr_sg4_multi** out) {
+// one_group: the contexts (of one basis) share a launch, in FP64 unless all run in fixed point.
+static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int flags, bool one_group,
+                        evr_sg4_multi** out) {
   if (!out) return set_error(EVR_ERR_ARG, "multi_create: NULL output");
   *out = nullptr;
   if (n < 1 || !ctxs || !nrhs) return set_error(EVR_ERR_ARG, "multi_create: NULL argument or n < 1");
@@ -1623,11 +2032,15 @@ extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* 
   m->d_contrib.assign(n, nullptr);
   m->d_part.assign(n, nullptr);
   auto fail = [&](int rc) { free_multi(m); return rc; };
-  // Launch groups.  The contexts with D <= 6 run narrow in a launch of their
-  // own when their items fill enough waves and other contexts exist;
-  // otherwise one launch takes every context, in the geometry of the merged
-  // wide plan (wide; narrow if every D <= 6, else mid, once it has enough
-  // waves of items).
+  m->fx.resize(n);
+  bool all_fx = true;
+  for (int k = 0; k < n; ++k) all_fx = all_fx && ctxs[k]->fx;
+  for (int k = 0; k < n; ++k) m->fx[k] = one_group ? all_fx : ctxs[k]->fx;
+  // Launch groups, for the fixed-point contexts and for the others.  The
+  // contexts with D <= 6 run narrow in a launch of their own when their items
+  // fill enough waves and other contexts exist; otherwise one launch takes
+  // every context, in the geometry of the merged wide plan (wide; narrow if
+  // every D <= 6, else mid, once it has enough waves of items).
   std::vector<size_t> n_wide(n);
   for (int k = 0; k < n; ++k) {
     evr_sg4_ctx* c = ctxs[k];
@@ -1635,34 +2048,40 @@ extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* 
     std::vector<Item> items;
     std::vector<float> cost;
     long long need = 0;
-    plan_work(c, (nrhs[k] * c->nb0) << m->cshift, geo_smem_bytes(0) / 8, terms, items, cost, need);
+    plan_work(c, m->fx[k], (nrhs[k] * c->nb0) << m->cshift, geo_smem_bytes(0, m->fx[k]) / 8, c->rmax, terms, items,
+              cost, need);
     n_wide[k] = items.size();
   }
   const int sms = ctxs[0]->num_sms;
-  size_t small_items = 0, all_items = 0;
-  int dmax = 0, n_small = 0;
-  for (int k = 0; k < n; ++k) {
-    all_items += n_wide[k];
-    dmax = std::max(dmax, ctxs[k]->D);
-    if (ctxs[k]->D <= EVR_NARROW_FMAX) {
-      small_items += n_wide[k];
-      ++n_small;
-    }
-  }
   m->group.assign(n, 0);
-  if (n_small > 0 && n_small < n && choose_geo(EVR_NARROW_FMAX, small_items, sms) == 1) {
+  for (int kind = 1; kind >= 0; --kind) {
+    size_t small_items = 0, all_items = 0;
+    int dmax = 0, n_small = 0, n_kind = 0;
+    for (int k = 0; k < n; ++k) {
+      if (m->fx[k] != kind) continue;
+      ++n_kind;
+      all_items += n_wide[k];
+      dmax = std::max(dmax, ctxs[k]->D);
+      if (ctxs[k]->D <= EVR_NARROW_FMAX) {
+        small_items += n_wide[k];
+        ++n_small;
+      }
+    }
+    if (n_kind == 0) continue;
+    const int g0 = (int)m->groups.size();
+    const bool two = n_small > 0 && n_small < n_kind && choose_geo(EVR_NARROW_FMAX, small_items, sms) == 1;
     int dbig = 0;
-    for (int k = 0; k < n; ++k)
-      if (ctxs[k]->D > EVR_NARROW_FMAX) {
-        m->group[k] = 1;
+    for (int k = 0; k < n; ++k) {
+      if (m->fx[k] != kind) continue;
+      m->group[k] = g0;
+      if (two && ctxs[k]->D > EVR_NARROW_FMAX) {
+        m->group[k] = g0 + 1;
         dbig = std::max(dbig, ctxs[k]->D);
       }
-    m->groups.resize(2);
-    m->groups[0].geo = 1;
-    m->groups[1].geo = choose_geo(dbig, all_items - small_items, sms);
-  } else {
-    m->groups.resize(1);
-    m->groups[0].geo = choose_geo(dmax, all_items, sms);
+    }
+    m->groups.resize(g0 + (two ? 2 : 1));
+    m->groups[g0].geo = two ? 1 : choose_geo(dmax, all_items, sms);
+    if (two) m->groups[g0 + 1].geo = choose_geo(dbig, all_items - small_items, sms);
   }
   {  // each group split into launches of at most EVR_PB_LARGE contexts, in context order
     std::vector<MGroup> split;
@@ -1700,8 +2119,9 @@ extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* 
   std::vector<std::vector<float>> allcost(ng);
   long long scratch_doubles = 0;
   for (MGroup& g : m->groups) {
-    g.smem_doubles = geo_smem_bytes(g.geo) / 8;
-    g.grid = geo_ctas(g.geo) * sms;
+    const bool fx = m->fx[g.ctx_of[0]];
+    g.smem_doubles = geo_smem_bytes(g.geo, fx) / 8;
+    g.grid = launch_ctas(g.geo, fx) * sms;
   }
   for (int k = 0; k < n; ++k) {
     evr_sg4_ctx* c = ctxs[k];
@@ -1715,10 +2135,10 @@ extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* 
     std::vector<Item> items;
     std::vector<float> cost;
     long long need = 0;
-    plan_work(c, nv, g.smem_doubles, terms, items, cost, need);
-    if (need > g.smem_doubles) g.scratch_per_cta = std::max(g.scratch_per_cta, need);
+    plan_work(c, m->fx[k], nv, g.smem_doubles, c->rmax, terms, items, cost, need);
+    g.scratch_per_cta = std::max(g.scratch_per_cta, need);
     for (size_t q = 0; q < items.size(); ++q) {
-      all[gk].push_back(MItem{m->slot[k], items[q].term, items[q].rhs0, 0});
+      all[gk].push_back(MItem{m->slot[k], items[q].term, items[q].rhs0, items[q].r});
       allcost[gk].push_back(cost[q]);
     }
     if (cudaMalloc(&m->d_terms[k], terms.size() * sizeof(TermInfo)) != cudaSuccess ||
@@ -1753,6 +2173,11 @@ extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* 
   }
   *out = m;
   return EVR_OK;
+}
+
+extern "C" int evr_sg4_multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int flags,
+                                    evr_sg4_multi** out) {
+  return multi_create(n, ctxs, nrhs, flags, false, out);
 }
 
 extern "C" int evr_sg4_multi_groups(const evr_sg4_multi* m, int cap, int* n_groups, int* geo, long long* n_items) {
@@ -1792,7 +2217,7 @@ extern "C" int evr_sg4_multi_hpsi(evr_sg4_multi* m, const double* const* psi, co
   for (int k = 0; k < m->n; ++k) {
     evr_sg4_ctx* c = m->ctxs[k];
     if (!psi[k]) continue;  // context k is skipped in this call
-    if (!c->have_op || c->type != m->type[k] || nbuf_for(c) != m->nbuf[k] || c->streamed)
+    if (!c->have_op || c->type != m->type[k] || nbuf_for(c) != m->nbuf[k] || c->streamed || (m->fx[k] && !c->fx))
       return set_error(EVR_ERR_STATE, "multi_hpsi: the operator of context %d changed since multi_create", k);
     if (!hpsi[k] || ldpsi[k] < c->nvec || ldh[k] < c->nvec)
       return set_error(EVR_ERR_ARG, "multi_hpsi: bad output or leading dimension for context %d", k);
@@ -1802,7 +2227,8 @@ extern "C" int evr_sg4_multi_hpsi(evr_sg4_multi* m, const double* const* psi, co
     KParams& p = params[k];
     p = make_params(c, m->nrhs_v[k], m->cshift, psi[k], ldpsi[k] << m->cshift, hpsi[k], ldh[k] << m->cshift, 1.0);
     const MGroup& g = m->groups[m->group[k]];
-    p.transpose = m->transpose;
+    use_transpose(p, c, m->transpose);
+    p.fx = m->fx[k];
     p.smem_doubles = g.smem_doubles;  // the plan's geometry, not the context's own last plan
     p.terms = m->d_terms[k];
     p.contrib = m->d_contrib[k];
@@ -1858,7 +2284,8 @@ int evr::multi_bind(evr_sg4_multi* m, int slot, const double* const* psi, double
     KParams& p = params[k];
     p = make_params(c, m->nrhs_v[k], m->cshift, psi[k], c->nvec << m->cshift, hpsi[k], c->nvec << m->cshift, 1.0);
     const MGroup& g = m->groups[m->group[k]];
-    p.transpose = m->transpose;
+    use_transpose(p, c, m->transpose);
+    p.fx = m->fx[k];
     p.smem_doubles = g.smem_doubles;
     p.terms = m->d_terms[k];
     p.contrib = m->d_contrib[k];
@@ -1948,11 +2375,10 @@ int evr::bound_apply_create(evr_sg4_ctx* c, int nrhs, int transpose, const doubl
   b->nrhs_v = nrhs * c->nb0;
   std::vector<TermInfo> terms;
   std::vector<Item> items, sorted;
-  long long max_need = 0;
-  plan_sorted(c, b->nrhs_v, terms, items, sorted, max_need, b->geo);
-  const int smem_doubles = geo_smem_bytes(b->geo) / 8;
-  b->grid = geo_ctas(b->geo) * c->num_sms;
-  const long long per_cta = max_need > smem_doubles ? max_need : 0;
+  long long per_cta = 0;
+  plan_sorted(c, b->nrhs_v, terms, items, sorted, per_cta, b->geo);
+  const int smem_doubles = geo_smem_bytes(b->geo, c->fx) / 8;
+  b->grid = launch_ctas(b->geo, c->fx) * c->num_sms;
   auto fail = [&](const char* what) {
     cudaGetLastError();
     bound_apply_destroy(b);
@@ -1971,7 +2397,7 @@ int evr::bound_apply_create(evr_sg4_ctx* c, int nrhs, int transpose, const doubl
     return fail("upload failed");
   b->n_items = (int)sorted.size();
   KParams p = make_params(c, b->nrhs_v, 0, psi, b->ld, hpsi, b->ld, 1.0);
-  p.transpose = transpose ? 1 : 0;
+  use_transpose(p, c, transpose);
   p.terms = b->d_terms;
   p.smem_doubles = smem_doubles;
   p.contrib = b->d_contrib;
@@ -2050,7 +2476,7 @@ int evr::field_pair_create(evr_sg4_ctx* a, evr_sg4_ctx* b, int transpose, int nr
   evr_sg4_ctx* cs[2] = {a, b};
   const int nr[2] = {nrhs, nrhs};
   FieldPair* f = new FieldPair();
-  int rc = evr_sg4_multi_create(2, cs, nr, EVR_APPLY_COMPLEX | (transpose ? EVR_APPLY_TRANSPOSE : 0), &f->m);
+  int rc = multi_create(2, cs, nr, EVR_APPLY_COMPLEX | (transpose ? EVR_APPLY_TRANSPOSE : 0), true, &f->m);
   if (rc) {
     delete f;
     return rc;
@@ -2068,7 +2494,8 @@ int evr::field_pair_create(evr_sg4_ctx* a, evr_sg4_ctx* b, int transpose, int nr
   KParams* ps = f->ps;
   for (int k = 0; k < 2; ++k) {
     ps[k] = make_params(cs[k], 2 * nrhs, 1, f->x, 2 * a->N, nullptr, 2 * a->N, 1.0);
-    ps[k].transpose = m->transpose;
+    use_transpose(ps[k], cs[k], m->transpose);
+    ps[k].fx = m->fx[k];
     ps[k].smem_doubles = g.smem_doubles;
     ps[k].terms = m->d_terms[k];
     ps[k].contrib = m->d_contrib[k];
@@ -2355,7 +2782,7 @@ namespace evr {
 static std::string tune_key(const evr_sg4_ctx* c, int nrhs, int flags) {
   char k[160];
   snprintf(k, sizeof(k), "D%d_L%d_LB%d_T%d_NB0%d_N%lld_R%d_C%d_G%d", c->D, c->L, c->LB, c->type, c->nb0, c->N, nrhs,
-           (flags & EVR_APPLY_COMPLEX) ? 1 : 0, c->d_G ? 1 : 0);
+           (flags & EVR_APPLY_COMPLEX) ? 1 : 0, c->has_G ? 1 : 0);
   return k;
 }
 

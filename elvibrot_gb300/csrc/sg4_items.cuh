@@ -45,6 +45,19 @@ namespace evr {
 #define EVR_MID_CTAS 6
 #endif
 #define EVR_MID_FMAX 12
+// The fixed-point kernels have one shape for every geometry: six CTAs of 128
+// threads an SM (80 registers, 34.75 KB).  The item's phases end in barriers,
+// which other CTAs fill; measured on the 6-D benchmark (20 vectors, two columns
+// an item): six CTAs of 128 threads 3.20 ms, eight 3.39, five of 192 3.65, four
+// of 192 3.36, four of 256 3.65, three of 256 3.73, two of 512 4.45, two of 384
+// 4.34, and four of 128 with four columns an item 3.49, two of 256 with four
+// 3.88; the order is the same, within 5 %, on the 7-D and 8-D operators.
+#ifndef EVR_FX_CTAS
+#define EVR_FX_CTAS 6
+#endif
+#ifndef EVR_FX_THREADS
+#define EVR_FX_THREADS 128
+#endif
 #define EVR_BIG_WAVES 4
 #ifndef EVR_NARROW_INC
 #define EVR_NARROW_INC 0  // the narrow kernel takes the point digits from divisions
@@ -64,6 +77,12 @@ struct TermInfo {
   float cost;
   double w;           // WeightSG
   unsigned char l[EVR_MAXD];
+};
+
+// what the fixed-point items need of a term besides
+struct FxTerm {
+  double wf[2];       // WeightSG times the scales of the 1-D matrices (forward, transposed)
+  long long tile;     // first tile of 32 points in the fixed-point metric
 };
 
 // Modes in ascending (nq-nb)/(nb*nq), ties by index (the basis->grid order
@@ -90,12 +109,13 @@ static inline void mode_order(const int* nb, const int* nq, int D, int* ord) {
 struct Item {
   int term;
   int rhs0;
+  int r;  // right-hand sides of the block
 };
 
 // a work item of a launch: the context's slot in the launch's parameter
-// block, the Smolyak term and the first right-hand side of the block
+// block, the Smolyak term, the first right-hand side of the block and their number
 struct MItem {
-  int ctx, term, rhs0, pad;
+  int ctx, term, rhs0, r;
 };
 
 // 1-D matrices of (mode, level), row-major [nout][nin] for the kernel.
@@ -161,6 +181,16 @@ struct KParams {
   const T1Term* t1terms;     // [n_t1]
   const double* t1grid;      // their grids, sum_nq each
   int split;                 // mode passes: 0 per-pass choice, 1 one thread per fibre, 2 per output
+  int fx;                    // the items run in fixed point (sg4_fixed.cuh)
+  const FxTerm* fxterms;     // [nb_SG]
+  const int2* fxm;           // fixed-point 1-D matrices, at the offsets of mats
+  const int2* Gfx;           // fixed-point metric in tiles (fx_g_index): G_ij 2^(ed_i + ed_j - geg[term] + 58),
+                             // element i*D + j for output i, input j (its transpose for H^T)
+  long long tbase;           // tile of the first entry (term slices)
+  const int* geg;            // [nb_SG] its exponent per term
+  const int* ed;             // [D*Lp1] exponent of d1GG's scale per (mode, level)
+  const int* rs;             // [D*Lp1] type 1: row-sum bounds of F2_ii d2GG (in 2^28), 0: no such term
+  int eK;                    // type 1: exponent of F2_ii d2GG's scale
 };
 
 struct ItemShared {
@@ -1067,5 +1097,7 @@ extern const MultiEntry<EVR_PB_SMALL> multi_small_wide, multi_small_narrow, mult
 extern const MultiEntry<EVR_PB_SMALL> multi_small10_wide, multi_small10_narrow, multi_small10_mid;
 extern const MultiEntry<EVR_PB_SMALL> multi_small1g_wide, multi_small1g_narrow, multi_small1g_mid;
 extern const MultiEntry<EVR_PB_LARGE> multi_large_wide, multi_large_narrow, multi_large_mid;
+extern const MultiEntry<EVR_PB_SMALL> multi_fxsmall;  // in fixed point (sg4_items_fx.cu)
+extern const MultiEntry<EVR_PB_LARGE> multi_fxlarge;
 
 }  // namespace evr

@@ -1,0 +1,118 @@
+"""The items in block fixed point (sg4_fixed.cuh), at the sizes and values where
+they can go wrong, against the oracle: the smallest and largest terms and 1-D
+grids, odd numbers of columns, metrics that are not symmetric or spread too far
+for one exponent, steep potentials, and columns that the FP64 code takes over.
+
+The tolerance is the parity tolerance of every H.psi test (1e-12): each stage
+keeps 2^-55 of its largest value, a term runs at most 2 D + 3 <= 27 stages, and
+the alternating Smolyak weights amplify a term's error by less than 10^3.
+"""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+
+from elvibrot_gb300 import ParamOp, SG4Basis, sub_TabOpPsi
+from elvibrot_gb300.configs import make_model, random_psi
+from oracle.oracle import OracleSG4
+
+from test_gpu_parity import gpu_apply, oracle_for, rel_err
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+
+
+def need_cuda():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+
+
+@pytest.mark.parametrize("D,L,type_op,nrhs", [
+    (1, 0, 10, 1), (1, 9, 10, 3), (1, 14, 1, 2),      # one mode: nq 2 to 16
+    (2, 14, 10, 2), (3, 13, 1, 3), (2, 0, 1, 5),      # the longest 1-D grids, the smallest terms
+    (4, 6, 10, 5), (5, 5, 10, 1), (6, 5, 10, 2),      # tiles of 32 points left partly empty
+    (7, 5, 10, 3), (9, 3, 10, 2), (12, 2, 10, 3),     # more modes than the register-resident sizes
+    (12, 2, 1, 2), (11, 3, 1, 1)])
+def test_fixed_point_matches_oracle(D, L, type_op, nrhs):
+    need_cuda()
+    m = make_model(D, L, type_op, 900 + 17 * D + L)
+    O, kw = oracle_for(m)
+    psi = random_psi(O.N, nrhs, 3)
+    e = rel_err(gpu_apply(m.operator(), psi), O.hpsi(psi, **kw))
+    print(f"D={D} L={L} type {type_op} nrhs={nrhs}: {e:.2e}")
+    assert e <= TOL
+
+
+def _grid_problem(D, L, seed):
+    b = SG4Basis(D, L, scaleQ=np.full(D, 0.4))
+    O = OracleSG4(D, L, L, 1, 1, 2, 1, scaleQ=np.full(D, 0.4))
+    return b, O, np.random.default_rng(seed)
+
+
+def test_metric_that_is_not_symmetric_and_its_transpose():
+    need_cuda()
+    b, O, rng = _grid_problem(5, 4, 11)
+    V, G = rng.normal(size=b.sum_nq), rng.normal(size=b.sum_nq * 25)
+    op = ParamOp(b, 10, V=V, G=G)
+    psi = random_psi(b.N, 3, 5)
+    H = O.hpsi(np.eye(b.N), type_op=10, V=V, G=G)
+    assert rel_err(gpu_apply(op, psi), H @ psi) <= TOL
+    P = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    out = torch.empty_like(P)
+    op.hpsi_dev(P, out, transpose=True)
+    assert rel_err(out.cpu().numpy().T, H.T @ psi) <= TOL
+
+
+@pytest.mark.parametrize("case", ["metric", "potential", "type0"])
+def test_fields_with_a_wide_range(case):
+    """A metric spread over 2^20 inside a term, and potentials that grow by 10^8 or
+    more towards the edge of the grid."""
+    need_cuda()
+    b, O, rng = _grid_problem(4, 6, 12)
+    r = np.abs(b.grid_points() * 0.4).max(axis=1)
+    G = rng.normal(size=b.sum_nq * 16) * 0.1 if case != "metric" else \
+        np.exp(rng.uniform(-7.0, 7.0, size=b.sum_nq * 16))
+    V = rng.normal(size=b.sum_nq) if case == "metric" else np.exp(6.0 * r * r)
+    t = 0 if case == "type0" else 10
+    kw = dict(V=V) if t == 0 else dict(V=V, G=G)
+    psi = random_psi(b.N, 3, 6)
+    assert rel_err(gpu_apply(ParamOp(b, t, **kw), psi), O.hpsi(psi, type_op=t, **kw)) <= TOL
+
+
+@pytest.mark.parametrize("type_op", [1, 10])
+def test_scaled_and_exceptional_columns(type_op):
+    """H (2^k x) = 2^k H x to the bit (one exponent per column), to rounding where
+    the FP64 code takes the column; a column that is not finite, or far from the
+    others in scale, leaves the others' bits alone."""
+    need_cuda()
+    m = make_model(4, 5, type_op, 31)
+    op = m.operator()
+    psi = random_psi(op.basis.N, 4, 8)
+    ref = gpu_apply(op, psi)
+    for k in (-250, -30, 1, 250):
+        assert np.array_equal(gpu_apply(op, np.ldexp(psi, k)), np.ldexp(ref, k))
+    for k in (-600, -310, 310, 600):
+        assert rel_err(np.ldexp(gpu_apply(op, np.ldexp(psi, k)), -k), ref) <= TOL
+    mixed = psi.copy()
+    mixed[:, 0] = np.ldexp(psi[:, 0], 700)
+    mixed[:, 2] = 0.0
+    mixed[3, 3] = np.inf
+    got = gpu_apply(op, mixed)
+    assert np.array_equal(got[:, 1], ref[:, 1])
+    assert rel_err(np.ldexp(got[:, 0], -700), ref[:, 0]) <= TOL
+    assert np.all(got[:, 2] == 0.0)
+    assert not np.all(np.isfinite(got[:, 3]))
+    mixed[3, 3] = np.nan
+    got = gpu_apply(op, mixed)
+    assert np.array_equal(got[:, 1], ref[:, 1]) and np.isnan(got[:, 3]).any()
+
+
+def test_complex_pair_shares_an_item():
+    need_cuda()
+    m = make_model(5, 4, 10, 33)
+    op = m.operator()
+    psi = random_psi(op.basis.N, 3, 9, complex_=True)
+    P = torch.from_numpy(np.ascontiguousarray(psi.T)).cuda()
+    got = sub_TabOpPsi(P, op).cpu().numpy().T
+    assert np.array_equal(got.real, gpu_apply(op, np.ascontiguousarray(psi.real)))
+    assert np.array_equal(got.imag, gpu_apply(op, np.ascontiguousarray(psi.imag)))
