@@ -388,8 +388,7 @@ __global__ void fields_kernel(const TermInfo* terms, long long nb_SG, const long
                               const int* nq_of_l, const double* xcat, const int* x_off, int D, int Lp1,
                               int V_nterms, const double* V_coef, const int* V_fac, double* V,
                               const double* G0, const double* G1, double* G, long long gp0, long long gp1, int nb0,
-                              long long vstride, int Gsym, int2* Gfx, const int* geg, const int* ed, const FxTerm* fxterms, long long tile0,
-                              int Gtr) {
+                              long long vstride, int Gsym) {
   for (long long gp = gp0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; gp < gp1;
        gp += (long long)gridDim.x * blockDim.x) {
     // binary search of the term owning global point gp
@@ -422,7 +421,7 @@ __global__ void fields_kernel(const TermInfo* terms, long long nb_SG, const long
         V[(long long)ab * vstride + gp - gp0] = v;
       }
     }
-    if (G || Gfx) {
+    if (G) {
       // a symmetric affine form (G0 and G1 symmetric in i, j, bit for bit)
       // gives G_ji the same FMA chain as G_ij: formed once, stored twice
       const long long nqt = T.nq;
@@ -433,17 +432,166 @@ __global__ void fields_kernel(const TermInfo* terms, long long nb_SG, const long
           if (G1)
             for (int k = 0; k < D; ++k) g = fma(G1[((long long)i * D + j) * D + k], Q[k], g);
           // GGiq(iq, j, i) of the term
-          if (G) {
-            G[o + nqt * ((long long)D * i + j)] = g;
-            if (Gsym) G[o + nqt * ((long long)D * j + i)] = g;
-          }
-          if (Gfx) {
-            const int2 f = fx_from(g, ed[i * Lp1 + T.l[i]] + ed[j * Lp1 + T.l[j]] - geg[lo] + 58);
-            const long long t0 = fxterms[lo].tile - tile0;
-            Gfx[fx_g_index(D, t0, (int)q, Gtr ? D * j + i : D * i + j)] = f;
-            if (Gsym) Gfx[fx_g_index(D, t0, (int)q, Gtr ? D * i + j : D * j + i)] = f;
-          }
+          G[o + nqt * ((long long)D * i + j)] = g;
+          if (Gsym) G[o + nqt * ((long long)D * j + i)] = g;
         }
+    }
+  }
+}
+
+// The same fields, one channel, from tables over two halves of the modes.
+// FP64 bounds fields_kernel: D products for each of the D^2 metric elements
+// of a point and every factor of every monomial.  A term's grid is a product,
+// q = (qA, qB) with qA the first h modes, so
+//   G(q) = GA(qA) + GB(qB),   V(q) = sum_m A_m(qA) W_m(qB),
+// A_m the distinct factors of the monomials over the first h modes and W_m
+// the rest of the monomials that share one, summed with their coefficients.  A
+// CTA takes one term and FS_NB values of qB, forms the tables in shared
+// memory FS_ITEMS elements or factors at a time, and combines them for its
+// points: an integer addition per metric element (both tables in fixed point
+// with the term's exponent, written as the items read them) and one FP64
+// multiply-add per factor.
+#define FS_THREADS 128
+#define FS_NA 64     // most qA (h: as many modes as fit, at least one; nq <= 16)
+#define FS_NB 32     // qB per CTA: a whole number of metric tiles
+#define FS_ITEMS 32  // elements or factors per table
+struct FieldUnit {
+  int term, b0;
+};
+// the monomials by their factors over the first h modes, h = 1..D
+struct VSplit {
+  int nterms;          // monomials
+  const int* a0;       // [D+1] first factor of split h at a0[h-1]
+  const int* afac;     // [factors][EVR_VFAC]
+  const int* bstart;   // first monomial of factor f of split h: bstart[a0[h-1] + h-1 + f]
+  const double* bcoef; // [D][nterms] coefficients, by factor
+  const int* bfac;     // [D][nterms][EVR_VFAC] what is left of each
+};
+struct FieldArgs {
+  const FieldUnit* units;
+  const TermInfo* terms;
+  const unsigned char* h;
+  const int* nq_of_l;
+  const double* xcat;
+  const int* x_off;
+  int D, Lp1;
+  VSplit vs;
+  double* V;
+  long long gp0;
+  const double *G0, *G1;
+  int2* Gfx;
+  const int *geg, *ed;
+  const FxTerm* fxterms;
+  long long tile0;
+  int Gtr;
+};
+
+// product of the factors f (mode << 8 | exponent, -1 ends) at the coordinates X[mode * stride]
+__device__ __forceinline__ double vfac_product(const int* f, const double* X, int stride, double m) {
+  for (int k = 0; k < EVR_VFAC && f[k] >= 0; ++k) {
+    const double x = X[(f[k] >> 8) * stride];
+    for (int e = 0; e < (f[k] & 255); ++e) m *= x;
+  }
+  return m;
+}
+
+__global__ void __launch_bounds__(FS_THREADS) fields_split_kernel(const __grid_constant__ FieldArgs p) {
+  __shared__ double XA[EVR_MAXD * FS_NA], XB[EVR_MAXD * FS_NB];
+  __shared__ double TA[FS_ITEMS * FS_NA], TB[FS_ITEMS * FS_NB];
+  const FieldUnit u = p.units[blockIdx.x];
+  const TermInfo& T = p.terms[u.term];
+  const int D = p.D, h = p.h[u.term], tid = threadIdx.x;
+  int nA = 1;
+  for (int i = 0; i < h; ++i) nA *= p.nq_of_l[i * p.Lp1 + T.l[i]];
+  const int nB = min(FS_NB, T.nq / nA - u.b0), npt = nA * nB, q0 = u.b0 * nA;
+  for (int e = tid; e < nA; e += FS_THREADS)
+    for (int i = 0, q = e; i < h; ++i) {
+      const int k = i * p.Lp1 + T.l[i], n = p.nq_of_l[k];
+      XA[i * FS_NA + e] = p.xcat[p.x_off[k] + q % n];
+      q /= n;
+    }
+  for (int e = tid; e < nB; e += FS_THREADS)
+    for (int i = h, q = u.b0 + e; i < D; ++i) {
+      const int k = i * p.Lp1 + T.l[i], n = p.nq_of_l[k];
+      XB[i * FS_NB + e] = p.xcat[p.x_off[k] + q % n];
+      q /= n;
+    }
+  __syncthreads();
+  if (p.V) {
+    constexpr int PT = FS_NA * FS_NB / FS_THREADS;
+    double v[PT];
+#pragma unroll
+    for (int k = 0; k < PT; ++k) v[k] = 0.0;
+    const int f0 = p.vs.a0[h - 1], nf = p.vs.a0[h] - f0;
+    const int* bs = p.vs.bstart + f0 + h - 1;
+    const double* bc = p.vs.bcoef + (long long)(h - 1) * p.vs.nterms;
+    const int* bf = p.vs.bfac + (long long)(h - 1) * p.vs.nterms * EVR_VFAC;
+    for (int m0 = 0; m0 < nf; m0 += FS_ITEMS) {
+      const int nm = min(FS_ITEMS, nf - m0);
+      for (int e = tid; e < nm * nA; e += FS_THREADS) {
+        const int m = e / nA, a = e - m * nA;
+        TA[m * FS_NA + a] = vfac_product(p.vs.afac + (long long)(f0 + m0 + m) * EVR_VFAC, XA + a, FS_NA, 1.0);
+      }
+      for (int e = tid; e < nm * nB; e += FS_THREADS) {
+        const int m = e / nB, b = e - m * nB;
+        double w = 0.0;
+        for (int t = bs[m0 + m]; t < bs[m0 + m + 1]; ++t)
+          w += vfac_product(bf + (long long)t * EVR_VFAC, XB + b, FS_NB, bc[t]);
+        TB[m * FS_NB + b] = w;
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < PT; ++k) {
+        const int e = tid + k * FS_THREADS;
+        if (e < npt) {
+          const int b = e / nA, a = e - b * nA;
+          for (int m = 0; m < nm; ++m) v[k] = fma(TA[m * FS_NA + a], TB[m * FS_NB + b], v[k]);
+        }
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int k = 0; k < PT; ++k)
+      if (tid + k * FS_THREADS < npt) p.V[T.off_nq - p.gp0 + q0 + tid + k * FS_THREADS] = v[k];
+  }
+  if (p.Gfx) {
+    long long *SA = reinterpret_cast<long long*>(TA), *SB = reinterpret_cast<long long*>(TB);
+    const int ne = D * D;
+    const long long tile = p.fxterms[u.term].tile - p.tile0 + q0 / FX_TILE;  // q0 is a multiple of the tile
+    int4* out = reinterpret_cast<int4*>(p.Gfx) + tile * (fx_tile_size(D) / 2);
+    for (int e0 = 0; e0 < ne; e0 += FS_ITEMS) {
+      const int nm = min(FS_ITEMS, ne - e0);
+      // part 0: G0 and the first h modes over qA; part 1: the other modes over qB
+      for (int part = 0; part < 2; ++part) {
+        const int n = part ? nB : nA, st = part ? FS_NB : FS_NA;
+        const double* X = part ? XB : XA;
+        for (int e = tid; e < nm * n; e += FS_THREADS) {
+          const int m = e / n, a = e - m * n;
+          int i = (e0 + m) / D, j = e0 + m - i * D;
+          if (p.Gtr) {
+            const int s = i;
+            i = j;
+            j = s;
+          }
+          double g = part ? 0.0 : (p.G0 ? p.G0[i * D + j] : (i == j ? 1.0 : 0.0));
+          if (p.G1)
+            for (int k = part ? h : 0; k < (part ? D : h); ++k)
+              g = fma(p.G1[((long long)i * D + j) * D + k], X[k * st + a], g);
+          const int s = p.ed[i * p.Lp1 + T.l[i]] + p.ed[j * p.Lp1 + T.l[j]] - p.geg[u.term] + 58;
+          (part ? SB : SA)[m * st + a] = __double2ll_rn(g * __hiloint2double((1023 + s) << 20, 0));
+        }
+      }
+      __syncthreads();
+      for (int e = tid; e < npt; e += FS_THREADS) {
+        const int b = e / nA, a = e - b * nA;
+        int4* o = out + (long long)(e / FX_TILE) * (fx_tile_size(D) / 2) + (e0 / 2) * FX_TILE + e % FX_TILE;
+        for (int m = 0; m < nm; m += 2, o += FX_TILE) {
+          const int2 x = fx_pack(SA[m * FS_NA + a] + SB[m * FS_NB + b]);
+          const int2 y = m + 1 < nm ? fx_pack(SA[(m + 1) * FS_NA + a] + SB[(m + 1) * FS_NB + b]) : make_int2(0, 0);
+          *o = make_int4(x.x, x.y, y.x, y.y);
+        }
+      }
+      __syncthreads();
     }
   }
 }
@@ -567,6 +715,12 @@ struct evr_sg4_ctx {
   double* d_G1 = nullptr;
   int G_sym = 0;                      // the affine G is symmetric bit for bit (G_ji formed once)
   long long* d_pt_start = nullptr;    // [nb_SG] first grid point of every term
+  // analytic fields of one channel from split tables (fields_split_kernel)
+  FieldUnit* d_units = nullptr;
+  std::vector<long long> unit_start;  // [nb_SG+1] first unit of every term
+  unsigned char* d_hsplit = nullptr;  // [nb_SG] modes in the first half
+  void* d_vsplit = nullptr;           // the VSplit arrays
+  VSplit vs = {};
   std::vector<long long> slice_term;  // [nslices+1] term ranges
   std::vector<int> slice_item;        // [nslices+1] ranges of the sorted work list
   // fixed-point items (sg4_fixed.cuh): the matrices and their scales, and
@@ -627,7 +781,7 @@ static void free_ctx(evr_sg4_ctx* c) {
                   c->d_scratch, c->d_V, c->d_G, c->d_Jac, c->d_cfac,
                   c->d_sqRho, c->d_F2, c->d_F1, c->d_io, c->d_Vcoef, c->d_Vfac, c->d_G0, c->d_G1,
                   c->d_pt_start, c->d_t1terms, c->d_t1grid, c->d_fxm, c->d_fxterms, c->d_ed, c->d_rs, c->d_geg, c->d_Gfx,
-                  c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT};
+                  c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT, c->d_units, c->d_hsplit, c->d_vsplit};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   delete c;
@@ -925,20 +1079,110 @@ extern "C" int evr_sg4_destroy(evr_sg4_ctx* c) {
   return EVR_OK;
 }
 
-// V (polynomial) and/or G (affine) on the grid points [g0, g1) (whole terms) into
-// the context's field arrays, from index 0.
-// transpose: the fixed-point metric of a streamed slice for H^T.
-static int eval_fields(evr_sg4_ctx* c, long long g0, long long g1, bool V, bool G, cudaStream_t s, long long tile0 = 0,
+// V (polynomial) and/or G (affine) on the terms [t0, t1) into the context's
+// field arrays, from index 0.  transpose: the fixed-point metric of a streamed
+// slice for H^T.
+static int eval_fields(evr_sg4_ctx* c, long long t0, long long t1, bool V, bool G, cudaStream_t s,
                        bool transpose = false) {
-  if (g1 <= g0) return EVR_OK;
-  const long long blocks = std::max<long long>(1, std::min<long long>((g1 - g0 + 255) / 256, 8LL * c->num_sms));
-  fields_kernel<<<(unsigned)blocks, 256, 0, s>>>(c->d_terms, c->nb_SG, c->d_pt_start, c->d_nq_of_l, c->d_x,
-                                                 c->d_x_off, c->D, c->L + 1, V ? c->V_nterms : 0, c->d_Vcoef,
-                                                 c->d_Vfac, V ? c->d_V : nullptr, c->d_G0, c->d_G1,
-                                                 G ? c->d_G : nullptr, g0, g1, c->nb0, c->z.sum_nq, c->G_sym,
-                                                 G ? c->d_Gfx : nullptr, c->d_geg, c->d_ed, c->d_fxterms, tile0,
-                                                 transpose);
+  if (t1 <= t0) return EVR_OK;
+  const long long g0 = c->terms[t0].off_nq, g1 = t1 < c->nb_SG ? c->terms[t1].off_nq : c->z.sum_nq;
+  const bool split = c->d_units != nullptr;  // one channel: V and the fixed-point metric
+  if (split && (V || (G && c->d_Gfx))) {
+    FieldArgs a = {};
+    a.units = c->d_units + c->unit_start[t0];
+    a.terms = c->d_terms;
+    a.h = c->d_hsplit;
+    a.nq_of_l = c->d_nq_of_l;
+    a.xcat = c->d_x;
+    a.x_off = c->d_x_off;
+    a.D = c->D;
+    a.Lp1 = c->L + 1;
+    a.vs = c->vs;
+    a.V = V ? c->d_V : nullptr;
+    a.gp0 = g0;
+    a.G0 = c->d_G0;
+    a.G1 = c->d_G1;
+    a.Gfx = G ? c->d_Gfx : nullptr;
+    a.geg = c->d_geg;
+    a.ed = c->d_ed;
+    a.fxterms = c->d_fxterms;
+    a.tile0 = a.Gfx ? c->fxterms[t0].tile : 0;
+    a.Gtr = transpose;
+    fields_split_kernel<<<(unsigned)(c->unit_start[t1] - c->unit_start[t0]), FS_THREADS, 0, s>>>(a);
+    V = false;
+  }
+  if (V || (G && c->d_G)) {
+    const long long blocks = std::max<long long>(1, std::min<long long>((g1 - g0 + 255) / 256, 8LL * c->num_sms));
+    fields_kernel<<<(unsigned)blocks, 256, 0, s>>>(c->d_terms, c->nb_SG, c->d_pt_start, c->d_nq_of_l, c->d_x,
+                                                   c->d_x_off, c->D, c->L + 1, V ? c->V_nterms : 0, c->d_Vcoef,
+                                                   c->d_Vfac, V ? c->d_V : nullptr, c->d_G0, c->d_G1,
+                                                   G ? c->d_G : nullptr, g0, g1, c->nb0, c->z.sum_nq, c->G_sym);
+  }
   CUDA_TRY(cudaGetLastError());
+  return EVR_OK;
+}
+
+// The units, splits and monomial tables of fields_split_kernel.
+static int split_fields(evr_sg4_ctx* c, const evr_sg4_op_desc* op, const std::vector<int>& vfac, bool polyV) {
+  const int D = c->D, nt = polyV ? op->V_nterms : 0;
+  std::vector<FieldUnit> units;
+  std::vector<unsigned char> hs(c->nb_SG);
+  c->unit_start.assign(1, 0);
+  for (long long t = 0; t < c->nb_SG; ++t) {
+    int h = 0, nA = 1;
+    while (h < D) {
+      const int n = c->nq_of_l[h * (c->L + 1) + c->terms[t].l[h]];
+      if (h > 0 && nA * n > FS_NA) break;
+      nA *= n;
+      ++h;
+    }
+    hs[t] = (unsigned char)h;
+    for (int b = 0; b < c->terms[t].nq / nA; b += FS_NB) units.push_back(FieldUnit{(int)t, b});
+    c->unit_start.push_back((long long)units.size());
+  }
+  int rc;
+  if ((rc = upload(&c->d_units, units.data(), units.size())) || (rc = upload(&c->d_hsplit, hs.data(), hs.size())))
+    return rc;
+  c->vs = VSplit{};
+  if (nt == 0) return EVR_OK;
+  std::vector<int> a0(1, 0), afac, bstart, bfac((size_t)D * nt * EVR_VFAC, -1);
+  std::vector<double> bcoef((size_t)D * nt);
+  for (int h = 1; h <= D; ++h) {
+    // each monomial's factors are in ascending mode order: those of modes < h
+    // come first; monomials ordered by them, in their own order within
+    std::vector<std::vector<int>> key(nt);
+    for (int k = 0; k < nt; ++k)
+      for (int f = 0; f < EVR_VFAC && vfac[(size_t)k * EVR_VFAC + f] >= 0; ++f)
+        if ((vfac[(size_t)k * EVR_VFAC + f] >> 8) < h) key[k].push_back(vfac[(size_t)k * EVR_VFAC + f]);
+    std::vector<int> ord(nt);
+    std::iota(ord.begin(), ord.end(), 0);
+    std::stable_sort(ord.begin(), ord.end(), [&](int x, int y) { return key[x] < key[y]; });
+    for (int r = 0; r < nt; ++r) {
+      const int k = ord[r];
+      if (r == 0 || key[k] != key[ord[r - 1]]) {
+        bstart.push_back(r);
+        for (int f = 0; f < EVR_VFAC; ++f) afac.push_back(f < (int)key[k].size() ? key[k][f] : -1);
+      }
+      bcoef[(size_t)(h - 1) * nt + r] = op->V_coef[k];
+      for (int f = (int)key[k].size(); f < EVR_VFAC; ++f)
+        bfac[((size_t)(h - 1) * nt + r) * EVR_VFAC + f - key[k].size()] = vfac[(size_t)k * EVR_VFAC + f];
+    }
+    bstart.push_back(nt);
+    a0.push_back((int)(afac.size() / EVR_VFAC));
+  }
+  // one allocation: the coefficients, then the integer tables
+  std::vector<int> all;
+  const size_t o1 = a0.size(), o2 = o1 + afac.size(), o3 = o2 + bstart.size();
+  all.insert(all.end(), a0.begin(), a0.end());
+  all.insert(all.end(), afac.begin(), afac.end());
+  all.insert(all.end(), bstart.begin(), bstart.end());
+  all.insert(all.end(), bfac.begin(), bfac.end());
+  CUDA_TRY(cudaMalloc(&c->d_vsplit, bcoef.size() * 8 + all.size() * 4));
+  double* bc = (double*)c->d_vsplit;
+  int* ip = (int*)(bc + bcoef.size());
+  CUDA_TRY(cudaMemcpy(bc, bcoef.data(), bcoef.size() * 8, cudaMemcpyHostToDevice));
+  CUDA_TRY(cudaMemcpy(ip, all.data(), all.size() * 4, cudaMemcpyHostToDevice));
+  c->vs = VSplit{nt, ip, ip + o1, ip + o2, bc, ip + o3};
   return EVR_OK;
 }
 
@@ -1103,10 +1347,14 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       cudaFree(*p);
       *p = nullptr;
     }
-  void* fxp[] = {c->d_rs, c->d_geg, c->d_Gfx, c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT};
+  void* fxp[] = {c->d_rs,    c->d_geg,    c->d_Gfx, c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT,
+                 c->d_units, c->d_hsplit, c->d_vsplit};
   for (void* q : fxp)
     if (q) cudaFree(q);
   c->d_rs = c->d_geg = nullptr;
+  c->d_units = nullptr;
+  c->d_hsplit = nullptr;
+  c->d_vsplit = nullptr;
   c->d_Gfx = c->d_GfxT = nullptr;
   c->fx = c->has_G = false;
   if (c->d_t1terms) cudaFree(c->d_t1terms);
@@ -1295,8 +1543,9 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
     }
     if (affG && op->G0 && (rc = upload(&c->d_G0, op->G0, (size_t)D * D))) return rc;
     if (affG && op->G1 && (rc = upload(&c->d_G1, op->G1, (size_t)D * D * D))) return rc;
+    if (c->nb0 == 1 && (polyV || (affG && fx)) && (rc = split_fields(c, op, vfac, polyV))) return rc;
     if (!stream) {
-      if ((rc = eval_fields(c, 0, snq, polyV, affG, 0))) return rc;
+      if ((rc = eval_fields(c, 0, c->nb_SG, polyV, affG, 0))) return rc;
       CUDA_TRY(cudaDeviceSynchronize());
     }
   }
@@ -1577,13 +1826,11 @@ static int hpsi_common(evr_sg4_ctx* c, int nrhs, int cshift, const double* psi, 
   if (!plain && c->streamed) {  // per slice: its fields, then its items
     for (size_t k = 0; k + 1 < c->slice_term.size(); ++k) {
       const long long t0 = c->slice_term[k], t1 = c->slice_term[k + 1];
-      const long long g0 = c->terms[t0].off_nq, g1 = t1 < c->nb_SG ? c->terms[t1].off_nq : c->z.sum_nq;
-      const long long tile0 = c->fxterms.empty() ? 0 : c->fxterms[t0].tile;
-      if ((rc = eval_fields(c, g0, g1, c->V_nterms > 0, c->d_G1 || c->d_G0, s, tile0, transpose))) return rc;
+      if ((rc = eval_fields(c, t0, t1, c->V_nterms > 0, c->d_G1 || c->d_G0, s, transpose))) return rc;
       CUDA_TRY(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned int), s));
       KParams q = p;
-      q.fbase = g0;
-      q.tbase = tile0;
+      q.fbase = c->terms[t0].off_nq;
+      q.tbase = c->fxterms.empty() ? 0 : c->fxterms[t0].tile;
       launch_single(c->geo, c->grid, smem, s, q, c->d_items + c->slice_item[k],
                     c->slice_item[k + 1] - c->slice_item[k], c->d_counter);
       CUDA_TRY(cudaGetLastError());

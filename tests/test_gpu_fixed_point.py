@@ -12,7 +12,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from elvibrot_gb300 import ParamOp, SG4Basis, sub_TabOpPsi
+from elvibrot_gb300 import ParamOp, Polynomial, SG4Basis, sub_TabOpPsi
 from elvibrot_gb300.configs import make_model, random_psi
 from oracle.oracle import OracleSG4
 
@@ -116,3 +116,28 @@ def test_complex_pair_shares_an_item():
     got = sub_TabOpPsi(P, op).cpu().numpy().T
     assert np.array_equal(got.real, gpu_apply(op, np.ascontiguousarray(psi.real)))
     assert np.array_equal(got.imag, gpu_apply(op, np.ascontiguousarray(psi.imag)))
+
+
+@pytest.mark.parametrize("D,L,terms", [(1, 14, 5), (2, 14, 40), (3, 9, 70), (7, 3, 200)])
+def test_polynomial_fields_match_grids(D, L, terms):
+    """V from its monomials (tables over two halves of the modes: one mode, the
+    longest grids, more factors than a table holds) and a metric that is affine
+    and not symmetric, against the same fields given as grids; H^T as well."""
+    need_cuda()
+    b, O, rng = _grid_problem(D, L, 13)
+    Q = b.grid_points()
+    expo = rng.integers(0, 4, size=(terms, D)) * (rng.random((terms, D)) < min(1.0, 3.0 / D))
+    poly = Polynomial(rng.normal(size=terms) * 0.1 ** expo.sum(axis=1), expo.astype(np.int32))
+    G0, G1 = np.eye(D) + 0.1 * rng.normal(size=(D, D)), 0.02 * rng.normal(size=(D, D, D))
+    nq = np.prod(b.tables()[0] + 2, axis=1)
+    off = np.concatenate([[0], np.cumsum(nq)])
+    g = G0 + np.einsum("ijk,pk->pij", G1, Q)
+    G = np.concatenate([g[off[t]:off[t + 1]].transpose(1, 2, 0).ravel() for t in range(len(nq))])
+    P = torch.from_numpy(np.ascontiguousarray(random_psi(b.N, 2, 4).T)).cuda()
+    for tr in (False, True):
+        outs = []
+        for kw in (dict(V_poly=poly, G0=G0, G1=G1), dict(V=poly(Q), G=G)):
+            out = torch.empty_like(P)
+            ParamOp(b, 10, **kw).hpsi_dev(P, out, transpose=tr)
+            outs.append(out.cpu().numpy())
+        assert rel_err(outs[0], outs[1]) <= TOL
