@@ -222,32 +222,6 @@ static cudaError_t set_smem_attributes() {
   return e;
 }
 
-__device__ __forceinline__ void neumaier_add(double& s, double& c, double x) {
-  const double t = s + x;
-  c += (fabs(s) >= fabs(x)) ? ((s - t) + x) : ((x - t) + s);
-  s = t;
-}
-
-// Neumaier sum of contrib[inv_idx[q] * nrhs_v + v] over q in [q0, q1), in
-// order, with the indices and values loaded eight at a time ahead of the
-// additions (each value sits behind an index load: a short list is
-// latency-bound); the additions are those of the plain loop, in its order.
-__device__ __forceinline__ void chunk_sum(const double* __restrict__ contrib, const long long* __restrict__ inv_idx,
-                                          long long q0, long long q1, int nrhs_v, int v, double& s, double& c) {
-  long long q = q0;
-  for (; q + 8 <= q1; q += 8) {
-    long long id[8];
-    double x[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) id[k] = inv_idx[q + k];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) x[k] = contrib[id[k] * nrhs_v + v];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) neumaier_add(s, c, x[k]);
-  }
-  for (; q < q1; ++q) neumaier_add(s, c, contrib[inv_idx[q] * nrhs_v + v]);
-}
-
 __device__ __forceinline__ void out_value(double* hpsi, const double* psi, long long n, int v, int cshift,
                                           long long ldpsi, long long ldh, double sum, double E0, double Esc,
                                           int nb0, long long Nfun) {
@@ -264,43 +238,38 @@ __device__ __forceinline__ void out_value(double* hpsi, const double* psi, long 
 
 // hpsi(n, v) = (sum_t contrib(k_t(n), v) - E0 psi(n, v)) / Esc, the sum over
 // the terms holding packed function n (inv_ptr/inv_idx is the inverse of
-// tab_iB_OF_SRep_TO_iB, in Smolyak-term order), in two phases so no thread
-// runs a long serial chain (the ground state is held by every term).  Each
-// packed function's list is cut into at most EVR_RED_CHUNKS chunks of at
-// least 16 entries:
-//   phase 1: one thread per (chunk, right-hand side) adds its chunk in term
-//            order with Neumaier compensation -> (s, c) partials;
-//   phase 2: one thread per (function, right-hand side) joins its chunk
-//            partials in order with TwoSum and writes (sum - E0 psi)/Esc.
-// The chunking is fixed at set-up, so results are deterministic, and the
-// compensated sums keep them independent of the sign pattern of the Smolyak
-// weights.
-#define EVR_RED_CHUNKS 32
-__global__ void __launch_bounds__(256) hpsi_reduce_chunks_kernel(
-    const double* __restrict__ contrib, const long long* __restrict__ chunk_q, long long n_chunks,
-    const long long* __restrict__ inv_idx, int nrhs_v, double2* __restrict__ part) {
-  const long long total = n_chunks * nrhs_v;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const long long ch = t / nrhs_v;
-    const int v = (int)(t - ch * nrhs_v);
-    double s = 0.0, c = 0.0;
-    chunk_sum(contrib, inv_idx, chunk_q[ch], chunk_q[ch + 1], nrhs_v, v, s, c);
-    part[t] = make_double2(s, c);
-  }
+// tab_iB_OF_SRep_TO_iB), in two kernels: one block per function and group of cw
+// columns adds the contributions (sum_function), then one thread per value writes the result.
+// The field-driven sweeps run the first one for both operators of a stage and
+// fuse the second one into the stage's arithmetic.
+__global__ void __launch_bounds__(EVR_SUM_THREADS) hpsi_sum_kernel(const double* __restrict__ contrib,
+                                                                   const long long* __restrict__ inv_ptr,
+                                                                   const long long* __restrict__ inv_idx, int nrhs_v,
+                                                                   int cw, double* __restrict__ part) {
+  const long long n = blockIdx.x;
+  sum_function(contrib, inv_idx, inv_ptr[n], inv_ptr[n + 1], nrhs_v, blockIdx.y * cw, cw, part + n * nrhs_v);
 }
 
-__global__ void __launch_bounds__(256) hpsi_reduce_join_kernel(
-    const double2* __restrict__ part, const long long* __restrict__ fun_chunk, long long N, int nrhs_v, int cshift,
-    const double* psi, long long ldpsi, double* hpsi, long long ldh, double E0, double Esc, int nb0) {
+__global__ void __launch_bounds__(256) hpsi_out_kernel(const double* __restrict__ part, long long N, int nrhs_v,
+                                                       int cshift, const double* psi, long long ldpsi, double* hpsi,
+                                                       long long ldh, double E0, double Esc, int nb0) {
   const long long total = N * nrhs_v;
   for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
        t += (long long)gridDim.x * blockDim.x) {
     const long long n = t / nrhs_v;
     const int v = (int)(t - n * nrhs_v);
-    out_value(hpsi, psi, n, v, cshift, ldpsi, ldh, join_chunks(part, fun_chunk[n], fun_chunk[n + 1], nrhs_v, v), E0,
-              Esc, nb0, N);
+    out_value(hpsi, psi, n, v, cshift, ldpsi, ldh, part[t], E0, Esc, nb0, N);
   }
+}
+
+// Columns of a block of the sums, a power of two: up to four, whose values fill
+// a 32-byte sector.  More of them would leave too few threads for the longest
+// list (the ground state is in every term): 32 took 170 us longer on the 6-D
+// benchmark (20 columns, lists of up to 2975).
+static int sum_columns(int nrhs_v) {
+  int cw = nrhs_v > 2 ? 4 : nrhs_v;
+  while (cw < 32 && (nrhs_v + cw - 1) / cw > 65535) cw *= 2;  // a grid's second dimension
+  return cw;
 }
 
 // Operator fields on the term grids: V from a polynomial, G from the affine
@@ -672,10 +641,7 @@ struct evr_sg4_ctx {
   unsigned int* d_counter = nullptr;
   long long* d_inv_ptr = nullptr;    // [N+1] packed function -> contributions
   long long* d_inv_idx = nullptr;    // [count(map>0)] global DP indices, term order
-  long long* d_chunk_q = nullptr;    // [n_chunks+1] list positions where chunks start
-  long long* d_fun_chunk = nullptr;  // [N+1] first chunk of every packed function
-  long long n_chunks = 0;
-  double* d_part = nullptr;          // [n_chunks][nrhs_v] chunk partials (s, c)
+  double* d_part = nullptr;          // [N][nrhs_v] sums
   size_t part_cap = 0;
   double* d_contrib = nullptr;       // [sum_nb][nrhs_v]
   size_t contrib_cap = 0;
@@ -777,7 +743,7 @@ static int nbuf_for(const evr_sg4_ctx* c) {
 static void free_ctx(evr_sg4_ctx* c) {
   void* ptrs[] = {c->d_map, c->d_mats, c->d_mat_off, c->d_diag_off, c->d_nb_of_l, c->d_nq_of_l, c->d_x, c->d_x_off,
                   c->d_terms, c->d_items, c->d_plain_items, c->d_counter, c->d_inv_ptr,
-                  c->d_inv_idx, c->d_contrib, c->d_chunk_q, c->d_fun_chunk, c->d_part,
+                  c->d_inv_idx, c->d_contrib, c->d_part,
                   c->d_scratch, c->d_V, c->d_G, c->d_Jac, c->d_cfac,
                   c->d_sqRho, c->d_F2, c->d_F1, c->d_io, c->d_Vcoef, c->d_Vfac, c->d_G0, c->d_G1,
                   c->d_pt_start, c->d_t1terms, c->d_t1grid, c->d_fxm, c->d_fxterms, c->d_ed, c->d_rs, c->d_geg, c->d_Gfx,
@@ -1023,17 +989,6 @@ extern "C" int evr_sg4_create(const evr_sg4_desc* d, evr_sg4_ctx** out) {
     for (long long k = 0; k < z.sum_nb; ++k)
       if (d->map[k] > 0) inv_idx[fill[d->map[k] - 1]++] = k;
   }
-  // chunks of each function's contribution list: at most EVR_RED_CHUNKS per function
-  std::vector<long long> chunk_q, fun_chunk(d->N + 1, 0);
-  for (long long n = 0; n < d->N; ++n) {
-    fun_chunk[n] = (long long)chunk_q.size();
-    const long long len = inv_ptr[n + 1] - inv_ptr[n];
-    const long long csz = std::max<long long>(16, (len + EVR_RED_CHUNKS - 1) / EVR_RED_CHUNKS);
-    for (long long q = inv_ptr[n]; q < inv_ptr[n + 1]; q += csz) chunk_q.push_back(q);
-  }
-  fun_chunk[d->N] = (long long)chunk_q.size();
-  c->n_chunks = (long long)chunk_q.size();
-  chunk_q.push_back(inv_ptr[d->N]);
   // launch geometry: persistent CTAs per SM sharing ~220 KB of shared memory
   // (wide until a work plan chooses otherwise)
   c->geo = 0;
@@ -1051,9 +1006,7 @@ extern "C" int evr_sg4_create(const evr_sg4_desc* d, evr_sg4_ctx** out) {
       (rc = upload<TermInfo>(&c->d_terms, nullptr, c->terms.size())) ||
       (rc = upload<unsigned int>(&c->d_counter, nullptr, 1)) ||
       (rc = upload(&c->d_inv_ptr, inv_ptr.data(), inv_ptr.size())) ||
-      (rc = upload(&c->d_inv_idx, inv_idx.data(), inv_idx.size())) ||
-      (rc = upload(&c->d_chunk_q, chunk_q.data(), chunk_q.size())) ||
-      (rc = upload(&c->d_fun_chunk, fun_chunk.data(), fun_chunk.size()))) {
+      (rc = upload(&c->d_inv_idx, inv_idx.data(), inv_idx.size()))) {
     free_ctx(c);
     return rc;
   }
@@ -1702,7 +1655,7 @@ static int build_items(evr_sg4_ctx* c, int nrhs_v) {
     c->scratch_cap = (size_t)per_cta * c->grid;
   }
   c->scratch_per_cta = per_cta;
-  size_t pneed = (size_t)c->n_chunks * nrhs_v * 2;
+  size_t pneed = (size_t)c->N * nrhs_v;
   if (pneed > c->part_cap) {
     if (c->d_part) cudaFree(c->d_part);
     c->d_part = nullptr;
@@ -1720,19 +1673,15 @@ static int build_items(evr_sg4_ctx* c, int nrhs_v) {
   return EVR_OK;
 }
 
-static int launch_reduce(evr_sg4_ctx* c, const double* contrib, double2* part, int nrhs_v, int cshift,
+static int launch_reduce(evr_sg4_ctx* c, const double* contrib, double* part, int nrhs_v, int cshift,
                          const double* psi, long long ldpsi, double* hpsi, long long ldh, double E0, double Esc,
                          cudaStream_t s) {
-  // 64-thread blocks, up to 64 per SM: every thread runs a serial chain of
-  // FP64 additions, and GB300's FP64 pipe (about two operations per clock
-  // per SM) wants small reductions spread over all SMs
-  const long long t1 = c->n_chunks * nrhs_v, t2 = c->N * nrhs_v;
-  const long long b1 = std::max<long long>(1, std::min<long long>((t1 + 63) / 64, 64LL * c->num_sms));
+  const long long t2 = c->N * nrhs_v;
   const long long b2 = std::max<long long>(1, std::min<long long>((t2 + 63) / 64, 64LL * c->num_sms));
-  hpsi_reduce_chunks_kernel<<<(unsigned)b1, 64, 0, s>>>(contrib, c->d_chunk_q, c->n_chunks, c->d_inv_idx, nrhs_v,
-                                                       part);
-  hpsi_reduce_join_kernel<<<(unsigned)b2, 64, 0, s>>>(part, c->d_fun_chunk, c->N, nrhs_v, cshift, psi, ldpsi, hpsi,
-                                                     ldh, E0, Esc, c->nb0);
+  const int cw = sum_columns(nrhs_v);
+  hpsi_sum_kernel<<<dim3((unsigned)c->N, (nrhs_v + cw - 1) / cw), EVR_SUM_THREADS, 0, s>>>(
+      contrib, c->d_inv_ptr, c->d_inv_idx, nrhs_v, cw, part);
+  hpsi_out_kernel<<<(unsigned)b2, 64, 0, s>>>(part, c->N, nrhs_v, cshift, psi, ldpsi, hpsi, ldh, E0, Esc, c->nb0);
   CUDA_TRY(cudaGetLastError());
   return EVR_OK;
 }
@@ -1849,7 +1798,7 @@ static int hpsi_common(evr_sg4_ctx* c, int nrhs, int cshift, const double* psi, 
     }
     CUDA_TRY(cudaGetLastError());
   }
-  if ((rc = launch_reduce(c, c->d_contrib, (double2*)c->d_part, nrhs_v, cshift, psi, ldv_psi, hpsi, ldv_h, E0, Esc,
+  if ((rc = launch_reduce(c, c->d_contrib, c->d_part, nrhs_v, cshift, psi, ldv_psi, hpsi, ldv_h, E0, Esc,
                           s)))
     return rc;
   CUDA_TRY(cudaGetLastError());
@@ -2081,7 +2030,7 @@ extern "C" int evr_probe_fp64_pipes(double* dfma_tflops, double* dmma_tflops, do
 // out of the driver's allocator, whose calls can synchronise the device.
 // evr_sg4_hpsi_noalloc gives them the persistent kernel with all of its scratch
 // -- the work counter, the term table of this call's plan, the work list,
-// the per-term contributions, the chunk partials of the ordered accumulation
+// the per-term contributions, the sums of the accumulation
 // and the per-CTA slabs for terms larger than shared memory -- carved from
 // one fixed, file-scope device array instead of device allocations.
 //
@@ -2145,7 +2094,7 @@ extern "C" int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi,
   int geo = 0;
   plan_sorted(c, nrhs_v, terms, items, sorted, per_cta, geo);
   int smem_doubles = geo_smem_bytes(geo, c->fx) / 8;
-  // carve: [counter | terms | items | contributions | chunk partials | large-term slabs], 256-byte aligned
+  // carve: [counter | terms | items | contributions | sums | large-term slabs], 256-byte aligned
   auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
   size_t off_terms, off_items, off_contrib, off_part, off_slabs, total;
   int grid;
@@ -2154,7 +2103,7 @@ extern "C" int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi,
     off_items = off_terms + up(terms.size() * sizeof(TermInfo));
     off_contrib = off_items + up(sorted.size() * sizeof(MItem));
     off_part = off_contrib + up((size_t)c->z.sum_nb * nrhs_v * 8);
-    off_slabs = off_part + up((size_t)c->n_chunks * nrhs_v * 16);
+    off_slabs = off_part + up((size_t)c->N * nrhs_v * 8);
     // with large-term slabs, launch only as many CTAs as the array has slabs for
     grid = launch_ctas(geo, c->fx) * c->num_sms;
     if (per_cta > 0 && off_slabs < (size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES)
@@ -2189,7 +2138,7 @@ extern "C" int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi,
   launch_single(geo, grid, (size_t)smem_doubles * 8, s, p, (const MItem*)(base + off_items), (int)ms.size(),
                 (unsigned int*)base);
   CUDA_TRY(cudaGetLastError());
-  int rc = launch_reduce(c, p.contrib, (double2*)(base + off_part), nrhs_v, 0, psi, ldpsi, hpsi, ldh, E0, Esc, s);
+  int rc = launch_reduce(c, p.contrib, (double*)(base + off_part), nrhs_v, 0, psi, ldpsi, hpsi, ldh, E0, Esc, s);
   if (rc) return rc;
   CUDA_TRY(cudaGetLastError());
   c->last_launches = 3;
@@ -2199,7 +2148,7 @@ extern "C" int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi,
 // ------------------------------------------------------------------------
 // Several independent Hamiltonians in one persistent launch.  The plan owns
 // everything that depends on the right-hand-side count (term blocks, the
-// per-term contributions, chunk partials, one global-scratch slab per CTA
+// per-term contributions, sums, one global-scratch slab per CTA
 // shared by all contexts) and the merged cost-sorted item list; the contexts
 // lend their read-only tables and operator grids.
 // ------------------------------------------------------------------------
@@ -2391,7 +2340,7 @@ static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int fl
     if (cudaMalloc(&m->d_terms[k], terms.size() * sizeof(TermInfo)) != cudaSuccess ||
         cudaMemcpy(m->d_terms[k], terms.data(), terms.size() * sizeof(TermInfo), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMalloc(&m->d_contrib[k], (size_t)c->z.sum_nb * nv * 8) != cudaSuccess ||
-        cudaMalloc(&m->d_part[k], (size_t)c->n_chunks * nv * 16) != cudaSuccess) {
+        cudaMalloc(&m->d_part[k], (size_t)c->N * nv * 8) != cudaSuccess) {
       cudaGetLastError();
       return fail(set_error(EVR_ERR_CUDA, "multi_create: device allocation for context %d failed", k));
     }
@@ -2507,7 +2456,7 @@ extern "C" int evr_sg4_multi_hpsi(evr_sg4_multi* m, const double* const* psi, co
   }
   for (int k = 0; k < m->n; ++k) {
     if (!psi[k]) continue;
-    int rc = launch_reduce(m->ctxs[k], m->d_contrib[k], (double2*)m->d_part[k], m->nrhs_v[k], m->cshift, psi[k],
+    int rc = launch_reduce(m->ctxs[k], m->d_contrib[k], m->d_part[k], m->nrhs_v[k], m->cshift, psi[k],
                            ldpsi[k] << m->cshift, hpsi[k], ldh[k] << m->cshift, E0 ? E0[k] : 0.0,
                            Esc ? Esc[k] : 1.0, s);
     if (rc) return rc;
@@ -2555,7 +2504,7 @@ int evr::multi_launch_bound(evr_sg4_multi* m, int slot, const double* const* psi
   }
   for (int k = 0; k < m->n; ++k) {
     const long long ld = m->ctxs[k]->nvec << m->cshift;
-    int rc = launch_reduce(m->ctxs[k], m->d_contrib[k], (double2*)m->d_part[k], m->nrhs_v[k], m->cshift, psi[k], ld,
+    int rc = launch_reduce(m->ctxs[k], m->d_contrib[k], m->d_part[k], m->nrhs_v[k], m->cshift, psi[k], ld,
                            hpsi[k], ld, E0[k], Esc[k], s);
     if (rc) return rc;
   }
@@ -2635,7 +2584,7 @@ int evr::bound_apply_create(evr_sg4_ctx* c, int nrhs, int transpose, const doubl
       cudaMalloc(&b->d_items, std::max<size_t>(1, sorted.size()) * sizeof(MItem)) != cudaSuccess ||
       cudaMalloc(&b->d_counter, sizeof(unsigned int)) != cudaSuccess ||
       cudaMalloc(&b->d_contrib, (size_t)c->z.sum_nb * b->nrhs_v * 8) != cudaSuccess ||
-      cudaMalloc(&b->d_part, (size_t)c->n_chunks * b->nrhs_v * 16) != cudaSuccess ||
+      cudaMalloc(&b->d_part, (size_t)c->N * b->nrhs_v * 8) != cudaSuccess ||
       (per_cta && cudaMalloc(&b->d_scratch, (size_t)per_cta * b->grid * 8) != cudaSuccess))
     return fail("device allocation failed");
   if (cudaMemcpy(b->d_terms, terms.data(), terms.size() * sizeof(TermInfo), cudaMemcpyHostToDevice) != cudaSuccess ||
@@ -2668,56 +2617,47 @@ int evr::bound_apply_launch(BoundApply* b, void* stream) {
   CUDA_TRY(cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned int), s));
   launch_single(b->geo, b->grid, (size_t)b->p.smem_doubles * 8, s, b->p, b->d_items, b->n_items, b->d_counter);
   CUDA_TRY(cudaGetLastError());
-  return launch_reduce(b->c, b->d_contrib, (double2*)b->d_part, b->nrhs_v, 0, b->psi, b->ld, b->hpsi, b->ld, 0.0,
+  return launch_reduce(b->c, b->d_contrib, b->d_part, b->nrhs_v, 0, b->psi, b->ld, b->hpsi, b->ld, 0.0,
                        1.0, s);
 }
 
 // ------------------------------------------------------------------------
 // Two operators of one basis (H0 and mu of a field-driven propagation)
-// applied to one complex vector in one persistent launch, up to the chunk
-// partials of their ordered accumulations; the caller joins them (and fuses
-// its own element-wise update into that join).  The parameter blocks point
+// applied to one complex vector in one persistent launch, up to the sums
+// of their accumulations; the caller reads them (and fuses its own
+// element-wise update into that).  The parameter blocks point
 // at a vector owned by the pair, so an apply uploads nothing and launches
-// two kernels: the merged item list, then the chunk sums of both operators
+// two kernels: the merged item list, then the sums of both operators
 // (which also rearms the work counter).
 // ------------------------------------------------------------------------
 struct evr::FieldPair {
   evr_sg4_multi* m = nullptr;
   double* x = nullptr;         // [nrhs][N] complex input
-  double2* part = nullptr;     // [2][n_chunks][2 nrhs]
+  double* part = nullptr;      // [2][N][2 nrhs] sums of both operators
   int grid = 0;
   int nrhs = 1;
   long long N = 0;
   KParams ps[2];               // the pair's parameters (slots 0 and 1 of its one launch group)
 };
 
-// Chunk sums of both operators: thread t = (op, chunk, virtual column v),
-// op-major, then chunk, then column (nrhs_v = 2 nrhs: re/im of each packet).
-__global__ void __launch_bounds__(256) pair_chunks_kernel(const double* __restrict__ contrib0,
-                                                          const double* __restrict__ contrib1,
-                                                          const long long* __restrict__ chunk_q, long long n_chunks,
-                                                          const long long* __restrict__ inv_idx, int nrhs_v,
-                                                          double2* __restrict__ part, unsigned int* counter) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) *counter = 0u;  // the item kernel before this one has finished
-  const long long per = n_chunks * nrhs_v, total = 2 * per;
-  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-       t += (long long)gridDim.x * blockDim.x) {
-    const int op = t >= per ? 1 : 0;
-    const long long r = t - op * per;
-    const long long ch = r / nrhs_v;
-    const int v = (int)(r - ch * nrhs_v);
-    const double* contrib = op ? contrib1 : contrib0;
-    double s = 0.0, c = 0.0;
-    chunk_sum(contrib, inv_idx, chunk_q[ch], chunk_q[ch + 1], nrhs_v, v, s, c);
-    part[t] = make_double2(s, c);
-  }
+// The sums of both operators: block (n, column group, op).
+__global__ void __launch_bounds__(EVR_SUM_THREADS) pair_sum_kernel(const double* __restrict__ contrib0,
+                                                                   const double* __restrict__ contrib1,
+                                                                   const long long* __restrict__ inv_ptr,
+                                                                   const long long* __restrict__ inv_idx, int nrhs_v,
+                                                                   int cw, double* __restrict__ part,
+                                                                   unsigned int* counter) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0) *counter = 0u;  // the item kernel has finished
+  const long long n = blockIdx.x, N = gridDim.x;
+  sum_function(blockIdx.z ? contrib1 : contrib0, inv_idx, inv_ptr[n], inv_ptr[n + 1], nrhs_v, blockIdx.y * cw, cw,
+               part + (blockIdx.z * N + n) * nrhs_v);
 }
 
 int evr::field_pair_create(evr_sg4_ctx* a, evr_sg4_ctx* b, int transpose, int nrhs, FieldPair** out) {
   *out = nullptr;
   if (!a || !b) return set_error(EVR_ERR_ARG, "field pair: NULL context");
   if (nrhs < 1) return set_error(EVR_ERR_ARG, "field pair: nrhs < 1");
-  if (a->N != b->N || a->nb_SG != b->nb_SG || a->z.sum_nb != b->z.sum_nb || a->n_chunks != b->n_chunks)
+  if (a->N != b->N || a->nb_SG != b->nb_SG || a->z.sum_nb != b->z.sum_nb)
     return set_error(EVR_ERR_ARG, "field pair: the two operators are on different bases");
   if (a->nb0 != 1 || b->nb0 != 1) return set_error(EVR_ERR_ARG, "field pair: one channel (nb0 = 1) only");
   evr_sg4_ctx* cs[2] = {a, b};
@@ -2731,7 +2671,7 @@ int evr::field_pair_create(evr_sg4_ctx* a, evr_sg4_ctx* b, int transpose, int nr
   f->N = a->N;
   f->nrhs = nrhs;
   if (cudaMalloc(&f->x, (size_t)a->N * nrhs * 16) != cudaSuccess ||
-      cudaMalloc(&f->part, (size_t)a->n_chunks * 4 * nrhs * sizeof(double2)) != cudaSuccess) {
+      cudaMalloc(&f->part, (size_t)a->N * 4 * nrhs * 8) != cudaSuccess) {
     cudaGetLastError();
     field_pair_destroy(f);
     return set_error(EVR_ERR_CUDA, "field pair: device allocation failed");
@@ -2775,13 +2715,10 @@ int evr::field_pair_apply(FieldPair* f, void* stream) {
   const MGroup& g = m->groups[0];
   launch_multi(g.geo, f->grid, (size_t)g.smem_doubles * 8, s, f->ps, 2, g.d_items, (int)g.sorted.size(), 0,
                g.d_counter);
-  // 64-thread blocks: the Neumaier sums are FP64 chains, and GB300's FP64
-  // pipe (about two operations per clock per SM) wants them on many SMs
   const int nrhs_v = 2 * f->nrhs;
-  const long long t1 = c->n_chunks * 2 * nrhs_v;
-  const long long b1 = std::max<long long>(1, std::min<long long>((t1 + 63) / 64, 64LL * c->num_sms));
-  pair_chunks_kernel<<<(unsigned)b1, 64, 0, s>>>(m->d_contrib[0], m->d_contrib[1], c->d_chunk_q, c->n_chunks,
-                                                 c->d_inv_idx, nrhs_v, f->part, g.d_counter);
+  const int cw = sum_columns(nrhs_v);
+  pair_sum_kernel<<<dim3((unsigned)c->N, (nrhs_v + cw - 1) / cw, 2), EVR_SUM_THREADS, 0, s>>>(
+      m->d_contrib[0], m->d_contrib[1], c->d_inv_ptr, c->d_inv_idx, nrhs_v, cw, f->part, g.d_counter);
   CUDA_TRY(cudaGetLastError());
   return EVR_OK;
 }
@@ -2790,9 +2727,7 @@ evr::FieldPairView evr::field_pair_view(const FieldPair* f) {
   FieldPairView v;
   const evr_sg4_ctx* c = f->m->ctxs[0];
   v.N = f->N;
-  v.n_chunks = c->n_chunks;
   v.nrhs = f->nrhs;
-  v.fun_chunk = c->d_fun_chunk;
   v.part = f->part;
   v.x = f->x;
   return v;
@@ -2954,7 +2889,7 @@ extern "C" int evr_sg4_diagonal(evr_sg4_ctx* c, double* diag, void* stream) {
       if (q) cudaFree(q);
   };
   if (cudaMalloc(&d_contrib, (size_t)c->z.sum_nb * 8) != cudaSuccess ||
-      cudaMalloc(&d_part, (size_t)c->n_chunks * 16) != cudaSuccess ||
+      cudaMalloc(&d_part, (size_t)c->N * 8) != cudaSuccess ||
       (per_cta && cudaMalloc(&d_scratch, (size_t)per_cta * grid * 8) != cudaSuccess) ||
       cudaMalloc(&d_pats, pats.size() * sizeof(DiagPat)) != cudaSuccess ||
       cudaMalloc(&d_order, order.size() * sizeof(int)) != cudaSuccess ||
@@ -2978,7 +2913,7 @@ extern "C" int evr_sg4_diagonal(evr_sg4_ctx* c, double* diag, void* stream) {
   diag_kernel<<<grid, 128, (size_t)smem_doubles * 8, s>>>(p, c->d_diag_off, d_pats, (int)pats.size(), d_order,
                                                           (int)c->nb_SG, d_counter);
   cudaError_t e = cudaGetLastError();
-  int rc = e == cudaSuccess ? launch_reduce(c, d_contrib, (double2*)d_part, 1, 0, diag, c->N, diag, c->N, 0.0, 1.0, s)
+  int rc = e == cudaSuccess ? launch_reduce(c, d_contrib, d_part, 1, 0, diag, c->N, diag, c->N, 0.0, 1.0, s)
                             : set_error(EVR_ERR_CUDA, "diagonal: %s", cudaGetErrorString(e));
   if (!rc && cudaStreamSynchronize(s) != cudaSuccess) rc = set_error(EVR_ERR_CUDA, "diagonal: kernel failed");
   cleanup();

@@ -29,16 +29,14 @@ int set_error(int code, const char* fmt, ...);
 int desc_sizes(const evr_sg4_desc* d, DescSizes* z);
 
 // Two operators on one basis applied to nrhs complex vectors in one launch,
-// up to the chunk partials of both ordered accumulations (part: [2][n_chunks]
-// [2 nrhs] (s, c) pairs: operator 0 first, then chunk, then re/im of each
-// vector); `x` is the device input block (N x nrhs complex, ld N) of every
+// up to the sums of both accumulations (part: [2][N][2 nrhs]: operator 0
+// first, then packed function, then re/im of each vector); `x` is the device input block (N x nrhs complex, ld N) of every
 // apply.  `transpose` applies both transposed.
 struct FieldPair;
 struct FieldPairView {
-  long long N = 0, n_chunks = 0;
+  long long N = 0;
   int nrhs = 1;
-  const long long* fun_chunk = nullptr;  // [N+1] first chunk of each packed function
-  const void* part = nullptr;            // double2 partials
+  const double* part = nullptr;
   double* x = nullptr;
 };
 int field_pair_create(evr_sg4_ctx* a, evr_sg4_ctx* b, int transpose, int nrhs, FieldPair** out);

@@ -18,7 +18,6 @@
 
 #include "evr_sg4.h"
 #include "sg4_internal.h"
-#include "sg4_reduce.cuh"
 
 namespace evr {
 
@@ -902,7 +901,7 @@ extern "C" int evr_sg4_cheby_propagate(evr_sg4_ctx* c, const evr_cheby_opts* o, 
 //
 // Every kernel of a field interval takes the interval index from a device
 // counter (SweepCtl) instead of a launch argument, so one field interval --
-// nsub steps x 4 stages x (H0/mu launch, chunk sums, stage update), then the
+// nsub steps x 4 stages x (H0/mu launch, sums, stage update), then the
 // counter update -- is recorded once as a CUDA graph and replayed for every
 // interval; the eager path launches the same kernels in the same order.
 // ------------------------------------------------------------------------
@@ -916,12 +915,10 @@ struct SweepCtl {
 };
 
 // The two operators of a stage (H0 and mu, or both transposed) run in one
-// persistent launch (field_pair_apply); the kernels below join their chunk
-// partials in the same order as evr_sg4_hpsi and fuse the stage arithmetic.
+// persistent launch (field_pair_apply); the kernels below take their sums and
+// do the stage arithmetic.
 struct StageIn {
-  const double2* part;         // [2][n_chunks][nrhs_v] (s, c) partials, H0 first
-  const long long* fun_chunk;  // [N+1]
-  long long nch2;              // n_chunks * nrhs_v: offset of mu's partials
+  const double* part;          // [2][N][nrhs_v] sums, H0 first
   long long N;
   int nb, nrhs_v;              // packets, 2 nb virtual columns
   double2* x;                  // stage input [nb][N], overwritten by the next stage's input
@@ -941,13 +938,12 @@ __device__ __forceinline__ double2* rec_at(const StageIn& a, int k, int u, int s
   return a.rec + (size_t)(seg & 1) * a.seg_rec + (((size_t)(k - seg * a.C) * a.nsub + u) * 4 + (stage - 1)) * a.N * a.nb;
 }
 
-// The four ordered sums of element (n, packet b) -- H0 re, H0 im, mu re,
-// mu im -- are joined by four lanes of a warp, one sum each, and gathered
-// with shuffles: GB300's FP64 pipe does about two operations per clock per
-// SM, so these joins must be spread over many SMs (a block of 32 threads
-// handles 8 elements); with one thread per element and 256-thread blocks the
-// stage kernels of a small operator ran on two SMs and took longer than its
-// H.psi launch.  Each sum is the join of evr_sg4_hpsi in its order.  Call
+// The four sums of element (n, packet b) -- H0 re, H0 im, mu re, mu im -- are
+// loaded by four lanes of a warp and gathered with shuffles: GB300's FP64 pipe
+// does about two operations per clock per SM, so the stage arithmetic must be
+// spread over many SMs (a block of 32 threads handles 8 elements); with one
+// thread per element and 256-thread blocks the stage kernels of a small
+// operator ran on two SMs and took longer than its H.psi launch.  Call
 // from every lane of a warp with the same e0 (the first element of the
 // warp's eight); lane q of group g handles element e0 + g.
 __device__ __forceinline__ bool stage_sums4(const StageIn& a, long long e0, long long& e, int& b, double2& xv,
@@ -961,8 +957,7 @@ __device__ __forceinline__ bool stage_sums4(const StageIn& a, long long e0, long
   if (e < ne) {
     b = (int)(e / a.N);
     n = e - (long long)b * a.N;
-    const long long c0 = a.fun_chunk[n], c1 = a.fun_chunk[n + 1];
-    v = join_chunks(a.part + (q >> 1) * a.nch2, c0, c1, a.nrhs_v, 2 * b + (q & 1));
+    v = a.part[((q >> 1) * a.N + n) * a.nrhs_v + 2 * b + (q & 1)];
   }
   const double hr0 = __shfl_sync(0xffffffffu, v, lane & ~3), hi0 = __shfl_sync(0xffffffffu, v, (lane & ~3) | 1);
   mr = __shfl_sync(0xffffffffu, v, (lane & ~3) | 2);
@@ -1155,7 +1150,7 @@ static void sweep_init(Sweep& w, FieldPair* fp, SweepCtl* ctl, const double* Ede
   w.fp = fp;
   w.adjoint = adjoint;
   const double h = o->dt / o->nsub;
-  w.a = StageIn{(const double2*)v.part, v.fun_chunk, v.n_chunks * 2 * nb, v.N, nb, 2 * nb, (double2*)v.x,
+  w.a = StageIn{v.part, v.N, nb, 2 * nb, (double2*)v.x,
                 Edev, ctl, o->E0, h, o->checkpoint, o->nsub, nullptr, 0};
   w.cr = std::cos(o->E0 * h);
   w.ci = adjoint ? std::sin(o->E0 * h) : -std::sin(o->E0 * h);  // e^{+i E0 h} backward, e^{-i E0 h} forward

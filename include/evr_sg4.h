@@ -426,7 +426,7 @@ typedef struct {
                           (fcn_field's para_H%E0; mid-spectrum keeps RK4 stable) */
   int nsub;            /* RK4 steps per field interval (dt/nsub each, E held) */
   int no_graph;        /* 0: every field interval (nsub steps x 4 stages, each one H0/mu
-                          launch, one chunk-sum launch and one stage update) is recorded
+                          launch, one sum launch and one stage update) is recorded
                           once as a CUDA graph and replayed, the interval index kept on
                           the device; 1: the same kernels launched one by one (same bits) */
 } evr_rk4_opts;

@@ -141,3 +141,15 @@ def test_polynomial_fields_match_grids(D, L, terms):
             ParamOp(b, 10, **kw).hpsi_dev(P, out, transpose=tr)
             outs.append(out.cpu().numpy())
         assert rel_err(outs[0], outs[1]) <= TOL
+
+
+@pytest.mark.parametrize("nrhs", [2, 3, 5, 33, 70])
+def test_sums_do_not_depend_on_the_number_of_columns(nrhs):
+    """The accumulation groups columns (one, two, or four a block): every column has
+    the bits of its own call, with lists from one term to all of them."""
+    need_cuda()
+    op = make_model(4, 6, 1, 41).operator()
+    psi = random_psi(op.basis.N, nrhs, 10)
+    got = gpu_apply(op, psi)
+    for j in {0, 1, nrhs - 1}:
+        assert np.array_equal(got[:, j], gpu_apply(op, psi[:, j:j + 1])[:, 0])
