@@ -210,7 +210,7 @@ static int smem_slack(int geo, bool fx) {
 
 // dynamic shared memory per CTA: the SM's 228 KB split between the resident
 // CTAs, less the slack above, so all of them fit (54.75 KB wide, 26.5 KB
-// narrow, 35.75 KB mid, 34.75 KB in fixed point)
+// narrow, 35.75 KB mid, 29.5 KB in fixed point)
 static int geo_smem_bytes(int geo, bool fx) {
   return (228 * 1024 / launch_ctas(geo, fx) - smem_slack(geo, fx)) / 256 * 256;
 }

@@ -31,7 +31,8 @@ enum {
   FX_MAXD = 12,                 // modes
   FX_STAGES = 2 * FX_MAXD + 3,  // recorded magnitudes: gather, B->G passes, U, O, G->B passes
   FX_FLUSH = 24,                // products |xh ml| <= 2^58 an accumulator takes before it is folded
-  FX_TILE = 32                  // points per tile of the fixed-point metric
+  FX_TILE = 32,                 // points per tile of the fixed-point metric
+  FX_AHEAD = 4                  // loads ahead of their products from global scratch
 };
 
 // int2 values of one tile of the fixed-point metric: its D*D elements, rounded
@@ -308,33 +309,45 @@ __device__ __noinline__ void fx_pass(const KParams& p, const ItemShared& it, FxS
   fx_pass_n<0, C, SM>(p, it, fs, ps, nin, nout, M, si, so, in, out, kind);
 }
 
-// sum over a fibre: n products of a matrix row with the fibre's values
+// sum over a fibre: n products of a matrix row with the fibre's values.  Two
+// values are loaded ahead of their products, or four where they come from
+// global scratch (L2 latency): with four 2.82 ms on the 6-D benchmark, three
+// 2.87, two 3.00.
 template <int C, bool SM>
 __device__ __forceinline__ void fx_fibre(FxAcc (&s)[C], int row, const FxArr<C, SM>& a, int i0, int n, int sd) {
+  constexpr int U = SM ? 2 : FX_AHEAD;
   const int2* Ms = reinterpret_cast<const int2*>(fx_sm);
   int m = 0;
-  for (; m + 1 < n; m += 2, row += 2, i0 += 2 * sd) {
-    const int2 m0 = Ms[row], m1 = Ms[row + 1];
-    const FxVal<C> v0 = a.load(i0), v1 = a.load(i0 + sd);
+  for (; m + U <= n; m += U, row += U, i0 += U * sd) {
+    FxVal<C> v[U];
 #pragma unroll
-    for (int w = 0; w < C; ++w) {
-      fx_mac(s[w], v0.h[w], v0.l[w], m0);
-      fx_mac(s[w], v1.h[w], v1.l[w], m1);
+    for (int k = 0; k < U; ++k) v[k] = a.load(i0 + k * sd);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const int2 mm = Ms[row + k];
+#pragma unroll
+      for (int w = 0; w < C; ++w) fx_mac(s[w], v[k].h[w], v[k].l[w], mm);
     }
   }
-  if (m < n) {
-    const int2 m0 = Ms[row];
-    const FxVal<C> v0 = a.load(i0);
+  if (U == 2) {
+    if (m < n) {
+      const int2 m0 = Ms[row];
+      const FxVal<C> v0 = a.load(i0);
 #pragma unroll
-    for (int w = 0; w < C; ++w) fx_mac(s[w], v0.h[w], v0.l[w], m0);
+      for (int w = 0; w < C; ++w) fx_mac(s[w], v0.h[w], v0.l[w], m0);
+    }
+  } else if (m < n) {  // one to U - 1 left
+    FxVal<C> v[U - 1];
+#pragma unroll
+    for (int k = 0; k < U - 1; ++k) v[k] = a.load(m + k < n ? i0 + k * sd : i0);
+#pragma unroll
+    for (int k = 0; k < U - 1; ++k)
+      if (m + k < n) {
+        const int2 mm = Ms[row + k];
+#pragma unroll
+        for (int w = 0; w < C; ++w) fx_mac(s[w], v[k].h[w], v[k].l[w], mm);
+      }
   }
-}
-
-// A mode's nq, grid stride, matrix and magic, the same for every lane: through
-// a warp reduction, so that the compiler keeps them in uniform registers.
-__device__ __forceinline__ int4 fx_uniform(int4 v) {
-  return make_int4(__reduce_max_sync(0xffffffffu, v.x), __reduce_max_sync(0xffffffffu, v.y),
-                   __reduce_max_sync(0xffffffffu, v.z), (int)__reduce_max_sync(0xffffffffu, (unsigned)v.w));
 }
 
 // Type 10, pass A: phi_j = d_j x at every point, then U_i = sum_j G_ji phi_j.
@@ -350,17 +363,13 @@ __device__ __forceinline__ void fx_type10_a(const KParams& p, const ItemShared& 
     m[w] = 0;
   }
   const FxArr<C, SM> x = B.x();
-  constexpr bool UNI = DD <= 6;  // beyond, the registers go to phi
-  int4 mds[UNI ? DD : 1];
-#pragma unroll
-  for (int j = 0; j < (UNI ? DD : 0); ++j) mds[j] = fx_uniform(fs.md[j]);
   const int2* G0 = p.Gfx + fs.tile * fx_tile_size(DD) + 2 * (threadIdx.x & 31);
   for (int q = threadIdx.x; q < nqt; q += blockDim.x) {
     FxVal<C> phi[DD];
     unsigned rem = (unsigned)q;
 #pragma unroll
     for (int j = 0; j < DD; ++j) {
-      const int4 md = UNI ? mds[UNI ? j : 0] : fs.md[j];
+      const int4 md = fs.md[j];
       const unsigned quo = md.w ? __umulhi(rem, (unsigned)md.w) : rem;
       const int idx = (int)(rem - quo * (unsigned)md.x);
       rem = quo;

@@ -45,15 +45,17 @@ namespace evr {
 #define EVR_MID_CTAS 6
 #endif
 #define EVR_MID_FMAX 12
-// The fixed-point kernels have one shape for every geometry: six CTAs of 128
-// threads an SM (80 registers, 34.75 KB).  The item's phases end in barriers,
-// which other CTAs fill; measured on the 6-D benchmark (20 vectors, two columns
-// an item): six CTAs of 128 threads 3.20 ms, eight 3.39, five of 192 3.65, four
+// The fixed-point kernels have one shape for every geometry: seven CTAs of 128
+// threads an SM (72 registers, 29.5 KB).  The item's phases end in barriers,
+// which other CTAs fill.  Measured on the 6-D benchmark (20 vectors, two columns
+// an item): seven CTAs of 128 threads 2.82 ms, six 2.89, eight (64 registers,
+// spills) 3.52; in an earlier build, against six at 3.20: five of 192 3.65, four
 // of 192 3.36, four of 256 3.65, three of 256 3.73, two of 512 4.45, two of 384
-// 4.34, and four of 128 with four columns an item 3.49, two of 256 with four
-// 3.88; the order is the same, within 5 %, on the 7-D and 8-D operators.
+// 4.34, four of 128 with four columns an item 3.49, two of 256 with four 3.88.
+// The 7-D, 8-D and uneven operators gain 2-5 % from the seventh CTA, the 12-D
+// streamed one loses 8 % (registers).
 #ifndef EVR_FX_CTAS
-#define EVR_FX_CTAS 6
+#define EVR_FX_CTAS 7
 #endif
 #ifndef EVR_FX_THREADS
 #define EVR_FX_THREADS 128
