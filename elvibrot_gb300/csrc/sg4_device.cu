@@ -13,11 +13,12 @@
 // shared memory (x in shared memory and the rest in a per-CTA slab of global
 // scratch when a term does not fit), apply the 1-D matrices mode by mode
 // (fused grid passes for the operators), and write each term's weighted
-// result to a contribution buffer that two small kernels then sum per packed
-// function in Smolyak-term order (compensated, deterministic, no atomics).
+// result to a contribution buffer, which is then summed exactly per packed
+// function (sg4_reduce.cuh).  The contractions run in block fixed point on the
+// integer pipe where the operator allows it (sg4_fixed.cuh), else in FP64.
 // The contexts' parameters travel by value in the launch (a __grid_constant__
-// block).  GB300's FP64 pipe (~1.25 TFLOP/s measured) is the binding
-// resource, so the kernel is organised to keep it busy: several CTAs per SM
+// block).  GB300's FP64 pipe (~1.25 TFLOP/s measured) binds the FP64 items,
+// so their kernel is organised to keep it busy: several CTAs per SM
 // (four, six, or eight for D <= 6) so some compute while the others gather or
 // synchronise, right-hand sides grouped per item so the 1-D matrices and the
 // operator fields are loaded once per point for the group, and no FP64 work

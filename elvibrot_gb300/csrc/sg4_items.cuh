@@ -717,9 +717,9 @@ __device__ void type10_fused_dispatch(const KParams& p, const ItemShared& it, co
 }
 
 // The weighted term result WeightSG(l) * y_b goes to contrib[off_nb + k][v]
-// (no atomics); the two reduce kernels add the contributions of each packed
-// function in Smolyak-term order, as tabR_AT_iG_TO_tabPackedBasis
-// accumulates them (sub_module_basis_BtoG_GtoB_SG4.f90:1255-1294).
+// (no atomics); the contributions of each packed function are then added
+// (sg4_reduce.cuh), as tabR_AT_iG_TO_tabPackedBasis accumulates them
+// (sub_module_basis_BtoG_GtoB_SG4.f90:1255-1294).
 static __device__ void store_contrib(const KParams& p, const ItemShared& it, const double* yb) {
   const int nbt = it.nb_t;
   const double wt = it.w;

@@ -386,7 +386,8 @@ class ParamOp:
         return n.value
 
     def last_geometry(self):
-        """(geometry, CTAs per SM) of the current work plan: 0 wide, 1 narrow, 2 mid."""
+        """(geometry, CTAs per SM of its FP64 kernels) of the current work plan: 0 wide,
+        1 narrow, 2 mid.  Fixed-point items run seven CTAs per SM in every geometry."""
         g, c = ctypes.c_int(), ctypes.c_int()
         check(lib().evr_sg4_last_geometry(self._h, ctypes.byref(g), ctypes.byref(c)))
         return g.value, c.value
