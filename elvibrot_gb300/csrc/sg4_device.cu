@@ -186,12 +186,12 @@ static int launch_ctas(int geo, bool fx) { return fx ? EVR_FX_CTAS : geo_ctas(ge
 
 // Static shared memory plus the 1 KB the driver reserves per CTA, rounded up
 // to 256 bytes (queried once): the largest of a geometry's kernels, so all
-// of them keep the geometry's CTAs per SM.  Index 3: the fixed-point kernels.
-static int smem_slack(int geo, bool fx) {
+// of them keep the geometry's CTAs per SM.
+static int smem_slack(int geo) {
   static const std::vector<int> slack = [] {
-    std::vector<int> v(4, 4096);
-    size_t a = 0, b = 0, c = 0, d = 0;
+    std::vector<int> v(3, 4096);
     for (int g = 0; g < 3; ++g) {
+      size_t a = 0, b = 0, c = 0, d = 0;
       const GeoKernels& k = geo_kernels(g);
       if (k.small->static_smem(&a) != cudaSuccess || k.large->static_smem(&b) != cudaSuccess ||
           k.small10->static_smem(&c) != cudaSuccess || k.small1g->static_smem(&d) != cudaSuccess) {
@@ -200,20 +200,16 @@ static int smem_slack(int geo, bool fx) {
       }
       v[g] = (int)((std::max(std::max(a, b), std::max(c, d)) + 1024 + 255) / 256 * 256);
     }
-    if (multi_fxsmall.static_smem(&a) == cudaSuccess && multi_fxlarge.static_smem(&b) == cudaSuccess)
-      v[3] = (int)((std::max(a, b) + 1024 + 255) / 256 * 256);
-    else
-      cudaGetLastError();
     return v;
   }();
-  return slack[fx ? 3 : geo];
+  return slack[geo];
 }
 
 // dynamic shared memory per CTA: the SM's 228 KB split between the resident
 // CTAs, less the slack above, so all of them fit (54.75 KB wide, 26.5 KB
 // narrow, 35.75 KB mid, 29.5 KB in fixed point)
 static int geo_smem_bytes(int geo, bool fx) {
-  return (228 * 1024 / launch_ctas(geo, fx) - smem_slack(geo, fx)) / 256 * 256;
+  return fx ? EVR_FX_SMEM : (228 * 1024 / geo_ctas(geo) - smem_slack(geo)) / 256 * 256;
 }
 
 // dynamic shared memory of every geometry's kernels (set at context creation)
@@ -227,9 +223,12 @@ static cudaError_t set_smem_attributes() {
     if (e == cudaSuccess) e = k.small10->set_smem(bytes);
     if (e == cudaSuccess) e = k.small1g->set_smem(bytes);
   }
-  const int bytes = geo_smem_bytes(0, true);
-  if (e == cudaSuccess) e = multi_fxsmall.set_smem(bytes);
-  if (e == cudaSuccess) e = multi_fxlarge.set_smem(bytes);
+  size_t a = 0, b = 0;
+  if (e == cudaSuccess) e = multi_fxsmall.static_smem(&a);
+  if (e == cudaSuccess) e = multi_fxlarge.static_smem(&b);
+  if (e == cudaSuccess && std::max(a, b) > EVR_FX_STATIC_SMEM) e = cudaErrorInvalidConfiguration;
+  if (e == cudaSuccess) e = multi_fxsmall.set_smem(EVR_FX_SMEM);
+  if (e == cudaSuccess) e = multi_fxlarge.set_smem(EVR_FX_SMEM);
   return e;
 }
 
@@ -772,14 +771,31 @@ static int upload(T** dst, const T* src, size_t n) {
   return EVR_OK;
 }
 
-// int2 values of the 1-D matrices that a fixed-point item keeps in shared memory
-static long long fx_mats(const evr_sg4_ctx* c, const TermInfo& T) {
+// int2 values of the 1-D matrices that a fixed-point item keeps in shared
+// memory, on a term of levels l
+template <class T>
+static long long fx_mats(int D, int L, const int* nb_of_l, const int* nq_of_l, const T* l) {
   long long n = 0;
-  for (int i = 0; i < c->D; ++i) {
-    const int k = i * (c->L + 1) + T.l[i];
-    n += (long long)c->nq_of_l[k] * (2 * c->nb_of_l[k] + c->nq_of_l[k]);
+  for (int i = 0; i < D; ++i) {
+    const int k = i * (L + 1) + (int)l[i];
+    n += (long long)nq_of_l[k] * (2 * nb_of_l[k] + nq_of_l[k]);
   }
   return (n + 1) & ~1LL;
+}
+static long long fx_mats(const evr_sg4_ctx* c, const TermInfo& T) {
+  return fx_mats(c->D, c->L, c->nb_of_l.data(), c->nq_of_l.data(), T.l);
+}
+
+extern "C" int evr_sg4_fixed_room(const evr_sg4_desc* d, long long* need, long long* room) {
+  if (!need || !room) return set_error(EVR_ERR_ARG, "fixed_room: NULL output");
+  DescSizes z;
+  int rc = desc_sizes(d, &z);
+  if (rc) return rc;
+  *need = 0;
+  *room = EVR_FX_SMEM / (long long)sizeof(int2);
+  for (long long t = 0; t < d->nb_SG; ++t)
+    *need = std::max(*need, fx_mats(d->D, d->L, d->nb_of_l, d->nq_of_l, d->tab_l + t * d->D));
+  return EVR_OK;
 }
 
 // (hi + lo) 2^58 in two limbs, rounded once (|lo| <= ulp(hi))
@@ -840,7 +856,6 @@ static int fx_matrices(evr_sg4_ctx* c, const std::vector<double>& weight) {
     }
   }
   for (long long t = 0; t < c->nb_SG; ++t) {
-    if (fx_mats(c, c->terms[t]) > 4096) return 0;  // they stay in shared memory beside the work arrays
     // the products as double-double (Dekker): one rounding at the end
     for (int d = 0; d < 2; ++d) {
       double hi = weight[t], lo = 0.0;
@@ -1003,7 +1018,16 @@ extern "C" int evr_sg4_create(const evr_sg4_desc* d, evr_sg4_ctx** out) {
   // launch geometry: persistent CTAs per SM sharing ~220 KB of shared memory
   // (wide until a work plan chooses otherwise)
   c->geo = 0;
-  if (D > FX_MAXD || !fx_matrices(c, std::vector<double>(d->weight, d->weight + d->nb_SG))) c->fxm.clear();
+  // fixed point: every term's matrices fit in the shared memory that its kernels
+  // are launched with, else the FP64 items keep the basis
+  long long fx_need = 0, fx_room = 0;
+  if ((rc = evr_sg4_fixed_room(d, &fx_need, &fx_room))) {
+    free_ctx(c);
+    return rc;
+  }
+  if (D > FX_MAXD || fx_need > fx_room ||
+      !fx_matrices(c, std::vector<double>(d->weight, d->weight + d->nb_SG)))
+    c->fxm.clear();
   c->smem_doubles = geo_smem_bytes(0, false) / 8;
   c->grid = geo_ctas(0) * c->num_sms;
   if ((rc = upload(&c->d_map, d->map, (size_t)z.sum_nb)) ||

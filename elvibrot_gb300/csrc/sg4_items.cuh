@@ -60,6 +60,12 @@ namespace evr {
 #ifndef EVR_FX_THREADS
 #define EVR_FX_THREADS 128
 #endif
+// Static shared memory of the fixed-point kernels (checked when they are
+// compiled and when a context is created), and what is left of the SM's 228 KB
+// for a CTA's dynamic shared memory, less the 1 KB the driver reserves: a
+// term's 1-D matrices have to fit there whole.
+#define EVR_FX_STATIC_SMEM 2048
+#define EVR_FX_SMEM ((228 * 1024 / EVR_FX_CTAS - EVR_FX_STATIC_SMEM - 1024) / 256 * 256)
 #define EVR_BIG_WAVES 4
 #ifndef EVR_NARROW_INC
 #define EVR_NARROW_INC 0  // the narrow kernel takes the point digits from divisions

@@ -11,6 +11,9 @@ namespace evr {
 
 #define EVR_K_CAP (EVR_KIND == 1 ? EVR_PB_LARGE : EVR_PB_SMALL)
 
+// the kernel's `it`, `fs` and `next`
+static_assert(sizeof(ItemShared) + sizeof(FxShared) + sizeof(int) <= EVR_FX_STATIC_SMEM, "static shared memory of the items");
+
 // The same item loop as hpsi_items_kernel.
 template <int CAP>
 __global__ void __launch_bounds__(EVR_FX_THREADS, EVR_FX_CTAS) hpsi_fixed_kernel(const __grid_constant__ ParamBlock<CAP> P,

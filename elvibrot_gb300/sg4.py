@@ -104,6 +104,7 @@ def _declare(L):
     L.evr_sg4_last_error.restype = ctypes.c_char_p
     sig = {
         "evr_sg4_desc_sizes": [ctypes.POINTER(Desc), ctypes.POINTER(ll)],
+        "evr_sg4_fixed_room": [ctypes.POINTER(Desc), ctypes.POINTER(ll), ctypes.POINTER(ll)],
         "evr_sg4_basis_build_ho": [ctypes.c_int] * 7 + [dp, dp, ctypes.POINTER(vp)],
         "evr_sg4_basis_build_ho_modes": [ctypes.c_int] * 3 + [ip] * 4 + [dp, dp, ctypes.POINTER(vp)],
         "evr_sg4_basis_desc": [vp, ctypes.POINTER(Desc)],

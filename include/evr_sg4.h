@@ -78,6 +78,10 @@ typedef struct {
 /* Sizes derived from a descriptor: out[0..7] = N, nb_SG, sum_nb, sum_nq,
  * max_nb_term, max_nq_term, D, L. */
 int evr_sg4_desc_sizes(const evr_sg4_desc* d, long long* out);
+/* Room for the 1-D matrices of one work item in fixed point, in 8-byte
+ * values: *need is what the basis' largest term takes, *room what a CTA has.
+ * A basis with need > room keeps the FP64 items.  Host only. */
+int evr_sg4_fixed_room(const evr_sg4_desc* d, long long* need, long long* room);
 
 /* ------------------------------------------------------------------------
  * Host builder for harmonic-oscillator (Hermite) primitive bases.

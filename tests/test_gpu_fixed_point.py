@@ -153,3 +153,16 @@ def test_sums_do_not_depend_on_the_number_of_columns(nrhs):
     got = gpu_apply(op, psi)
     for j in {0, 1, nrhs - 1}:
         assert np.array_equal(got[:, j], gpu_apply(op, psi[:, j:j + 1])[:, 0])
+
+
+@pytest.mark.parametrize("D,nb,nq", [(5, 16, 16), (4, 16, 16)])
+def test_long_grids_on_both_sides_of_the_shared_memory_bound(D, nb, nq):
+    """One term of D long 1-D grids: the five modes' matrices (3840 values) do not
+    fit in a fixed-point CTA, the four modes' ones (3072) do."""
+    need_cuda()
+    b = SG4Basis(D, 0, A_nb=nb, A_nq=nq, scaleQ=np.full(D, 0.5))
+    O = OracleSG4(D, 0, 0, nb, 0, nq, 0, scaleQ=np.full(D, 0.5))
+    Q = O.grid_points()
+    V, F2 = 0.1 * (Q * Q).sum(axis=1), -0.5 * np.eye(D)
+    psi = random_psi(b.N, 1, 21)
+    assert rel_err(gpu_apply(ParamOp(b, 1, V=V, F2=F2), psi), O.hpsi(psi, type_op=1, V=V, F2=F2)) <= TOL

@@ -71,3 +71,19 @@ def test_weights_sum_to_one_and_map_covers_packed_basis():
         tl, w, m = Bs.tables()
         assert abs(w.sum() - 1.0) < 1e-12
         assert set(m[m > 0]) == set(range(1, Bs.N + 1))
+
+
+@pytest.mark.parametrize("D,nb,nq,fits", [(5, 16, 16, False), (6, 14, 15, False), (6, 12, 16, False),
+                                          (7, 13, 14, False), (4, 16, 16, True), (6, 14, 14, True),
+                                          (7, 12, 14, True), (5, 15, 16, True), (1, 1, 1, True)])
+def test_fixed_point_matrices_fit_in_a_ctas_shared_memory(D, nb, nq, fits):
+    """An item in fixed point keeps its term's 1-D matrices (nq (2 nb + nq) values a
+    mode) in the CTA's dynamic shared memory: seven CTAs share the SM's 228 KB, less
+    2 KB of static memory and the driver's 1 KB each."""
+    need, room = ctypes.c_longlong(), ctypes.c_longlong()
+    b = SG4Basis(D, 0, A_nb=nb, A_nq=nq)
+    assert lib().evr_sg4_fixed_room(ctypes.byref(b.desc), ctypes.byref(need), ctypes.byref(room)) == 0
+    values = D * nq * (2 * nb + nq)
+    assert need.value == values + values % 2
+    assert room.value * 8 <= 228 * 1024 // 7 - 2048 - 1024
+    assert (need.value <= room.value) == fits
