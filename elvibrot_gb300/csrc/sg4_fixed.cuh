@@ -16,11 +16,11 @@
 // result (two to four), not the product of all of them.  That keeps 55 to 57
 // bits of each stage's largest value, against the 53 of a double.
 //
-// A right-hand side whose largest entry lies outside 2^+-300, or is not
-// finite, and one whose V.x is tiny against max|V| max|x| (a potential so
-// steep that the tails of x carry it), goes through the FP64 item code
-// instead, that column alone.  Operators the scheme does not suit (see
-// fx_prepare in sg4_device.cu) never come here.
+// A right-hand side whose largest entry in a term lies outside 2^+-300 (all
+// subnormal, for instance), or is not finite, and one whose V.x is tiny against
+// max|V| max|x| (a potential so steep that the tails of x carry it), goes
+// through the FP64 item code instead, that column alone.  Operators the scheme
+// does not suit (see fx_prepare in sg4_device.cu) never come here.
 #pragma once
 #include "sg4_items.cuh"
 
@@ -576,9 +576,10 @@ __device__ __forceinline__ void fx_body(const KParams& p, const ItemShared& it, 
 #pragma unroll
     for (int w = 0; w < C; ++w) {
       const long long b = *G0.raw(k, w);
+      if (em[w] == 0 && (b << 1) != 0) atomicOr(&fs.bad, 1 << w);  // subnormal entries alone
       const int e = (int)(b >> 52) & 0x7ff, s = em[w] - e;
       long long y = ((b & 0xFFFFFFFFFFFFFLL) | (e ? 0x10000000000000LL : 0)) << 6;
-      y = s > 60 || fx_bad_exp(em[w]) ? 0 : (s ? ((y >> (s - 1)) + 1) >> 1 : y);
+      y = s > 60 || em[w] == 0 || fx_bad_exp(em[w]) ? 0 : (s ? ((y >> (s - 1)) + 1) >> 1 : y);
       const int2 t = fx_pack(b < 0 ? -y : y);
       f.h[w] = t.x;
       f.l[w] = t.y;

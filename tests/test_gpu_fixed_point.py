@@ -166,3 +166,36 @@ def test_long_grids_on_both_sides_of_the_shared_memory_bound(D, nb, nq):
     V, F2 = 0.1 * (Q * Q).sum(axis=1), -0.5 * np.eye(D)
     psi = random_psi(b.N, 1, 21)
     assert rel_err(gpu_apply(ParamOp(b, 1, V=V, F2=F2), psi), O.hpsi(psi, type_op=1, V=V, F2=F2)) <= TOL
+
+
+@pytest.mark.parametrize("type_op", [1, 10])
+def test_subnormal_columns_and_blocks(type_op):
+    """A column that has decayed below 2^-1022 beside a normal one, as a real column
+    and as one part of a complex one; terms whose entries are all subnormal beside a
+    normal function that they do not hold; a block with one subnormal entry.  H is
+    linear, so the results are those of the scaled vectors, to the spacing of the
+    subnormal numbers (2^-1074) times the values that a result adds."""
+    need_cuda()
+    m = make_model(4, 5, type_op, 31)
+    op = m.operator()
+    psi = random_psi(op.basis.N, 3, 8)
+    ref = gpu_apply(op, psi)
+    tiny = np.ldexp(1.0, -1074)
+    x = psi.copy()
+    x[:, 0] = np.ldexp(psi[:, 0], -1040)                      # 2^-1040: 34 bits left
+    exact = np.ldexp(x[:, 0], 1040)                           # what those bits hold
+    got = gpu_apply(op, x)
+    assert np.array_equal(got[:, 1:], ref[:, 1:])
+    assert np.max(np.abs(np.ldexp(got[:, 0], 1040) - gpu_apply(op, exact[:, None])[:, 0])) <= 1e5 * np.ldexp(tiny, 1040)
+    z = psi[:, :1] + 1j * x[:, :1]
+    P = torch.from_numpy(np.ascontiguousarray(z.T)).cuda()
+    h = sub_TabOpPsi(P, op).cpu().numpy().T
+    assert np.array_equal(h.real, ref[:, :1]) and np.max(np.abs(h.imag)) < 1e-300
+    # one normal entry in the last function, 1e-310 elsewhere: H e_last everywhere
+    last = np.zeros((op.basis.N, 1))
+    last[-1] = 1.0
+    y = np.where(last == 0.0, 1e-310, last)
+    assert np.max(np.abs(gpu_apply(op, y) - gpu_apply(op, last))) < 1e-300
+    one = np.zeros((op.basis.N, 1))
+    one[0] = tiny
+    assert np.max(np.abs(gpu_apply(op, one))) <= 1e5 * tiny
