@@ -856,7 +856,7 @@ static int fx_matrices(evr_sg4_ctx* c, const std::vector<double>& weight) {
     }
   }
   for (long long t = 0; t < c->nb_SG; ++t) {
-    // the products as double-double (Dekker): one rounding at the end
+    // the products as double-double (Dekker)
     for (int d = 0; d < 2; ++d) {
       double hi = weight[t], lo = 0.0;
       for (int i = 0; i < D; ++i)
@@ -868,6 +868,7 @@ static int fx_matrices(evr_sg4_ctx* c, const std::vector<double>& weight) {
         }
       if (!(std::fabs(hi + lo) < 1e200)) return 0;
       c->fxterms[t].wf[d] = hi + lo;
+      c->fxterms[t].wl[d] = (hi - c->fxterms[t].wf[d]) + lo;
     }
     c->fxterms[t].tile = tile;
     tile += (c->terms[t].nq + FX_TILE - 1) / FX_TILE;

@@ -65,7 +65,7 @@ struct FxShared {
   int bad;                        // columns left to the FP64 code
   int msz;                        // int2 values of the term's matrices
   long long tile;                 // the term's first tile of the metric
-  double wf;                      // weight times the matrices' scales
+  double wf, wl;                  // weight times the matrices' scales, in two parts
 };
 
 // The item's matrices, then its work arrays x and U_1..U_D (type 10) or O.
@@ -253,9 +253,11 @@ __device__ __forceinline__ void fx_pass_n(const KParams& p, const ItemShared& it
       if (__ldg(p.map + it.off_nb + o) > 0) {
         double* cb = p.contrib + (it.off_nb + o) * p.nrhs_v + it.rhs0;
 #pragma unroll
-        for (int w = 0; w < C; ++w)
-          cb[w] = (double)(fx_sum(s[w], a[w]) - (1 << 28)) *
-                  (fs.wf * __hiloint2double((1023 + fs.eo[w] - a[w]) << 20, 0));
+        for (int w = 0; w < C; ++w) {
+          const double y = (double)(fx_sum(s[w], a[w]) - (1 << 28)) *
+                           __hiloint2double((1023 + fs.eo[w] - a[w]) << 20, 0);
+          cb[w] = fma(y, fs.wf, y * fs.wl);
+        }
       }
     } else {
       FxVal<C> y;
@@ -699,6 +701,7 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
     it.nq_t = T.nq;
     it.w = T.w;
     fs.wf = p.fxterms[term].wf[p.transpose];
+    fs.wl = p.fxterms[term].wl[p.transpose];
     fs.bad = 0;
     fs.evmax = 0;
     fs.rsum = 0;

@@ -89,7 +89,9 @@ struct TermInfo {
 
 // what the fixed-point items need of a term besides
 struct FxTerm {
-  double wf[2];       // WeightSG times the scales of the 1-D matrices (forward, transposed)
+  double wf[2];       // WeightSG times the scales of the 1-D matrices (forward, transposed) ...
+  double wl[2];       // ... and what its rounding left: one error shared by a whole term does not
+                      // average out in the alternating sum over the terms
   long long tile;     // first tile of 32 points in the fixed-point metric
 };
 

@@ -12,9 +12,9 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from elvibrot_gb300 import ParamOp, Polynomial, SG4Basis, sub_TabOpPsi
+from elvibrot_gb300 import ParamOp, Polynomial, SG4Basis, SG4Tables, sub_TabOpPsi
 from elvibrot_gb300.configs import make_model, random_psi
-from oracle.oracle import OracleSG4
+from oracle.oracle import OracleSG4, oracle_tables
 
 from test_gpu_parity import gpu_apply, oracle_for, rel_err
 
@@ -199,3 +199,72 @@ def test_subnormal_columns_and_blocks(type_op):
     one = np.zeros((op.basis.N, 1))
     one[0] = tiny
     assert np.max(np.abs(gpu_apply(op, one))) <= 1e5 * tiny
+
+
+# ------------------------------------------------------------- smooth vectors
+def _smooth_vectors(n):
+    """Columns that fall off with the excitation sum(n), and one that does not: N(0, 1)
+    entries times exp(-a sum(n)), the lowest function, a displaced ground state."""
+    rng = np.random.default_rng(1)
+    s = n.sum(axis=1)
+    r = rng.normal(size=len(s))
+    fact = np.cumprod(np.concatenate([[1.0], np.arange(1.0, n.max() + 1)]))
+    cols = [r, r * np.exp(-1.0 * s), r * np.exp(-3.0 * s), r * np.exp(-6.0 * s), (s == 0) * 1.0,
+            np.prod(0.7 ** n / np.sqrt(fact[n]), axis=1)]
+    return np.stack([c / np.linalg.norm(c) for c in cols], axis=1)
+
+
+def _metric(kind, Q, nq):
+    """GGiq(iq, j, i) per term of the identity times a factor of the point."""
+    D = Q.shape[1]
+    f = 1.0 + 0.05 * Q.sum(axis=1) if kind == "affine" else np.exp(kind * (Q * Q).sum(axis=1))
+    off = np.concatenate([[0], np.cumsum(nq)])
+    return np.concatenate([(np.eye(D)[:, :, None] * f[a:b]).ravel() for a, b in zip(off[:-1], off[1:])])
+
+
+POTENTIALS = {
+    "none": None,
+    "harmonic": lambda y: 0.5 * (y * y).sum(axis=1),
+    "quartic": lambda y: 0.5 * (y * y).sum(axis=1) + 0.1 * (y ** 4).sum(axis=1),
+    "morse": lambda y: ((1.0 - np.exp(-0.8 * y)) ** 2).sum(axis=1) / 1.28,
+    "wall": lambda y: np.exp(0.3 * (y * y).sum(axis=1)),
+}
+
+
+def _errors_in_both_arithmetics(D, L, type_op, pot, rules=(1, 1, 2, 1), metric="affine"):
+    """2-norm errors of each column against the long-double oracle, in fixed point and
+    from the FP64 items, which the same operator with a vanishing F1 term (types 0 and
+    1) or a unit Jacobian grid (type 10) keeps."""
+    O = OracleSG4(D, L, L, *rules)
+    T = SG4Tables(**oracle_tables(O))
+    tab_l, _, _, packed = O.tables()
+    Q, psi = O.grid_points(), _smooth_vectors(packed - 1)
+    kw = {} if POTENTIALS[pot] is None else dict(V=POTENTIALS[pot](Q))
+    if type_op == 1:
+        kw["F2"] = (-0.5 * np.eye(D)).ravel()
+    if type_op == 10:
+        kw["G"] = _metric(metric, Q, np.prod(tab_l * rules[3] + rules[2], axis=1))
+    ref = O.hpsi(psi, type_op=type_op, extended=True, **kw)
+    twin = dict(Jac=np.ones(O.sum_nq)) if type_op == 10 else dict(F1=np.full(D, 1e-300))
+    ops = ParamOp(T, type_op, **kw), ParamOp(T, 10 if type_op == 10 else 1, **kw, **twin)
+    return [np.linalg.norm(gpu_apply(op, psi) - ref, axis=0) / np.linalg.norm(ref, axis=0) for op in ops]
+
+
+def _no_less_precise(*args, **kw):
+    """Fixed point is no further from the exact result than the FP64 items: on the
+    geometric mean over the columns, and to a factor of four on any one of them (two
+    sums of rounding errors, each known to about a factor of two; half an ulp of the
+    result at least)."""
+    fx, f64 = _errors_in_both_arithmetics(*args, **kw)
+    r = np.maximum(fx, 2.0 ** -54) / np.maximum(f64, 2.0 ** -54)
+    print(args, kw, "fixed point / FP64:", np.round(r, 2), "mean %.2f" % np.exp(np.log(r).mean()))
+    assert np.exp(np.log(r).mean()) <= 1.0
+    assert r.max() <= 4.0
+
+
+@pytest.mark.parametrize("D,L,type_op,pot", [
+    (4, 8, 0, "harmonic"), (4, 8, 10, "harmonic"),   # one rounding shared by a term
+])
+def test_smooth_vectors_keep_their_digits(D, L, type_op, pot):
+    need_cuda()
+    _no_less_precise(D, L, type_op, pot)
