@@ -710,12 +710,11 @@ struct evr_sg4_ctx {
   std::vector<int> ed;                // [D*(L+1)] exponent of d1GG's scale
   int2* d_fxm = nullptr;
   int* d_ed = nullptr;
-  int* d_rs = nullptr;
+  int* d_e1 = nullptr;
   int* d_geg = nullptr;
   int2* d_Gfx = nullptr;
   int2* d_GfxT = nullptr;             // its transpose, for H^T (the same array when G is symmetric)
   long long all_tiles = 0, slice_tiles = 0;  // tiles of a resident metric; those allocated (the largest slice)
-  int eK = 0;
   // host-pointer path buffers
   double* d_io = nullptr;
   size_t io_cap = 0;
@@ -756,7 +755,7 @@ static void free_ctx(evr_sg4_ctx* c) {
                   c->d_inv_idx, c->d_contrib, c->d_part,
                   c->d_scratch, c->d_V, c->d_G, c->d_Jac, c->d_cfac,
                   c->d_sqRho, c->d_F2, c->d_F1, c->d_io, c->d_Vcoef, c->d_Vfac, c->d_G0, c->d_G1,
-                  c->d_pt_start, c->d_t1terms, c->d_t1grid, c->d_fxm, c->d_fxterms, c->d_ed, c->d_rs, c->d_geg, c->d_Gfx,
+                  c->d_pt_start, c->d_t1terms, c->d_t1grid, c->d_fxm, c->d_fxterms, c->d_ed, c->d_e1, c->d_geg, c->d_Gfx,
                   c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT, c->d_units, c->d_hsplit, c->d_vsplit};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -1230,22 +1229,30 @@ static bool fx_prepare(evr_sg4_ctx* c, const evr_sg4_op_desc* op, bool polyV, bo
       sum += big;
     }
     if (!inside(sum)) return false;
-    c->eK = sum > 0.0 ? std::ilogb(sum) + 1 : 0;
-    std::vector<int> rs((size_t)D * Lp1, 0);
+    // each matrix on a scale of its own; a term's items bring them to the
+    // scale of the term's sum (one scale for all terms would cost those of low
+    // levels up to seven bits of their kinetic energy)
+    std::vector<int> e1((size_t)D * Lp1, FX_NONE);
     for (int k = 0; k < D * Lp1; ++k) {
       const double f = c->F2[(k / Lp1) * (D + 1)];
-      if (f == 0.0) continue;
-      rs[k] = (int)std::ceil(std::ldexp(n[k], 30 - c->eK)) + 1;
+      if (n[k] == 0.0) continue;
+      e1[k] = std::ilogb(n[k]) + 1;
       for (int t = 0; t < 2; ++t) {
         const int o = c->mat_off[k * 8 + 4 * t + M_D2], nq = c->nq_of_l[k];
         for (int e = 0; e < nq * nq; ++e) {
           const double m = f * c->mats[o + e];
-          c->fxm[o + e] = fx_of(std::ldexp(m, -c->eK), std::ldexp(std::fma(f, c->mats[o + e], -m), -c->eK));
+          c->fxm[o + e] = fx_of(std::ldexp(m, -e1[k]), std::ldexp(std::fma(f, c->mats[o + e], -m), -e1[k]));
         }
       }
     }
+    geg.assign(c->nb_SG, 0);
+    for (long long t = 0; t < c->nb_SG; ++t) {
+      double s = 0.0;
+      for (int i = 0; i < D; ++i) s += n[i * Lp1 + c->terms[t].l[i]];
+      if (s > 0.0) geg[t] = std::ilogb(s) + 1;
+    }
     if (cudaMemcpy(c->d_fxm, c->fxm.data(), c->fxm.size() * sizeof(int2), cudaMemcpyHostToDevice) != cudaSuccess ||
-        upload(&c->d_rs, rs.data(), rs.size())) {
+        upload(&c->d_e1, e1.data(), e1.size())) {
       cudaGetLastError();
       return false;
     }
@@ -1336,11 +1343,11 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       cudaFree(*p);
       *p = nullptr;
     }
-  void* fxp[] = {c->d_rs,    c->d_geg,    c->d_Gfx, c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT,
+  void* fxp[] = {c->d_e1,    c->d_geg,    c->d_Gfx, c->d_GfxT == c->d_Gfx ? nullptr : c->d_GfxT,
                  c->d_units, c->d_hsplit, c->d_vsplit};
   for (void* q : fxp)
     if (q) cudaFree(q);
-  c->d_rs = c->d_geg = nullptr;
+  c->d_e1 = c->d_geg = nullptr;
   c->d_units = nullptr;
   c->d_hsplit = nullptr;
   c->d_vsplit = nullptr;
@@ -1425,6 +1432,7 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
   std::vector<int> geg;
   c->has_G = op->type == 10 && (op->G_grid || affG);
   bool fx = fx_prepare(c, op, polyV, affG, geg);
+  if (fx && !geg.empty() && (rc = upload(&c->d_geg, geg.data(), geg.size()))) return rc;
   if (polyV) CUDA_TRY(cudaMalloc(&c->d_V, (size_t)slice_pts * 8 * c->nb0 * c->nb0));
   if (op->type == 10) {
     if (op->G_grid) {
@@ -1438,7 +1446,6 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
         if (stream) return set_error(EVR_ERR_ALLOC, "set_operator: no memory for a slice of the metric");
         fx = false;
       }
-      if (fx && (rc = upload(&c->d_geg, geg.data(), geg.size()))) return rc;
     }
     if (op->Jac_grid) {
       for (long long k = 0; k < snq; ++k)
@@ -1769,8 +1776,7 @@ static KParams make_params(evr_sg4_ctx* c, int nrhs_v, int cshift, const double*
   p.Gfx = c->d_Gfx;  // use_transpose swaps it
   p.geg = c->d_geg;
   p.ed = c->d_ed;
-  p.rs = c->d_rs;
-  p.eK = c->eK;
+  p.e1 = c->d_e1;
   return p;
 }
 

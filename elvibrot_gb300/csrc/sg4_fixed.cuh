@@ -32,7 +32,8 @@ enum {
   FX_STAGES = 2 * FX_MAXD + 3,  // recorded magnitudes: gather, B->G passes, U, O, G->B passes
   FX_FLUSH = 24,                // products |xh ml| <= 2^58 an accumulator takes before it is folded
   FX_TILE = 32,                 // points per tile of the fixed-point metric
-  FX_AHEAD = 4                  // loads ahead of their products from global scratch
+  FX_AHEAD = 4,                 // loads ahead of their products from global scratch
+  FX_NONE = -(1 << 30)          // exponent of a type-1 mode without a derivative term
 };
 
 // int2 values of one tile of the fixed-point metric: its D*D elements, rounded
@@ -61,7 +62,7 @@ struct FxShared {
   int mv[FX_MAXR];                // largest bits(|h|) + biased exponent of V over the points
   int evmax;                      // largest biased exponent of V
   int e[FX_MAXR], eo[FX_MAXR];    // exponents of the running stage and of the grid result
-  int rsum;                       // type 1: sum of the term's derivative row sums (in 2^28)
+  int deriv;                      // type 1: some mode has a derivative term
   int bad;                        // columns left to the FP64 code
   int msz;                        // int2 values of the term's matrices
   long long tile;                 // the term's first tile of the metric
@@ -438,7 +439,7 @@ __device__ __noinline__ void fx_type10_a_dispatch(const KParams& p, const ItemSh
 template <int C, bool SM>
 __device__ __noinline__ void fx_grid(const KParams& p, const ItemShared& it, FxShared& fs, const FxBufs<C, SM> B) {
   const int D = p.D, nqt = it.nq_t;
-  const bool t10 = p.type == 10, hasT = t10 || fs.rsum > 0;
+  const bool t10 = p.type == 10, hasT = t10 || fs.deriv;
   int a[C], h[C], sP[C];
   unsigned m[C];
 #pragma unroll
@@ -452,8 +453,8 @@ __device__ __noinline__ void fx_grid(const KParams& p, const ItemShared& it, FxS
       eT = eX - aX + p.geg[it.term] - 1 - aT;
       if (fs.mx[D + 1][w]) bT = 59 + max(0, kD - aU) + eT;
     } else if (hasT) {
-      aT = min(28, aX + max(0, __clz(fs.rsum) - 2));
-      eT = eX + p.eK - aT;
+      aT = aX;
+      eT = eX + p.geg[it.term] - aT;
       if (fs.mx[D][w]) bT = 59 + eT;
     }
     const bool hasV = p.V && fs.mv[w] > 600;  // V x is there, and not below 2^-400
@@ -543,7 +544,15 @@ __device__ __forceinline__ void fx_body(const KParams& p, const ItemShared& it, 
     for (int i = tid >> 5; i < D; i += blockDim.x >> 5) {
       const int nbq = 2 * it.nb[i] * it.nq[i], nqq = it.nq[i] * it.nq[i];
       const int2 *s1 = p.fxm + it.mo[i][M_BG], *s2 = p.fxm + it.mo[i][p.type == 10 ? M_D1 : M_D2];
-      for (int e = tid & 31; e < nbq + nqq; e += 32) Ms[fs.moff[i] + e] = __ldg(e < nbq ? s1 + e : s2 + (e - nbq));
+      // type 1: the modes' derivative matrices, each kept on its own scale, go
+      // into one sum: onto the term's
+      const int sh = fs.deriv && fs.md[i].z >= 0
+                         ? min(p.geg[it.term] - p.e1[i * p.Lp1 + p.terms[it.term].l[i]], 62) : 0;
+      for (int e = tid & 31; e < nbq + nqq; e += 32) {
+        int2 m = __ldg(e < nbq ? s1 + e : s2 + (e - nbq));
+        if (sh > 0 && e >= nbq) m = fx_pack((((((long long)m.x << 29) + m.y) >> (sh - 1)) + 1) >> 1);
+        Ms[fs.moff[i] + e] = m;
+      }
     }
   }
   // gather (tabPackedBasis_TO_tabR_AT_iG) into the buffer from which the D
@@ -704,7 +713,7 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
     fs.wl = p.fxterms[term].wl[p.transpose];
     fs.bad = 0;
     fs.evmax = 0;
-    fs.rsum = 0;
+    fs.deriv = 0;
   }
   if (tid < D) {
     const int l = p.terms[term].l[tid];
@@ -753,9 +762,8 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
     int md = mo + 2 * di;
     if (i == D - 1) fs.msz = (md + it.nq[i] * it.nq[i] + 1) & ~1;
     if (p.type != 10) {
-      const int rs = p.type == 1 ? p.rs[i * p.Lp1 + p.terms[term].l[i]] : 0;
-      if (!rs) md = -1;
-      else atomicAdd(&fs.rsum, rs);
+      if (p.type == 1 && p.e1[i * p.Lp1 + p.terms[term].l[i]] != FX_NONE) fs.deriv = 1;
+      else md = -1;
     }
     fs.md[i] = make_int4(it.nq[i], st, md, (int)it.mg[i]);
   }

@@ -197,10 +197,9 @@ struct KParams {
   const int2* Gfx;           // fixed-point metric in tiles (fx_g_index): G_ij 2^(ed_i + ed_j - geg[term] + 58),
                              // element i*D + j for output i, input j (its transpose for H^T)
   long long tbase;           // tile of the first entry (term slices)
-  const int* geg;            // [nb_SG] its exponent per term
+  const int* geg;            // [nb_SG] its exponent per term; type 1: that of the term's sum of F2_ii d2GG
   const int* ed;             // [D*Lp1] exponent of d1GG's scale per (mode, level)
-  const int* rs;             // [D*Lp1] type 1: row-sum bounds of F2_ii d2GG (in 2^28), 0: no such term
-  int eK;                    // type 1: exponent of F2_ii d2GG's scale
+  const int* e1;             // [D*Lp1] type 1: that of F2_ii d2GG's scale, FX_NONE: no such term
 };
 
 struct ItemShared {
