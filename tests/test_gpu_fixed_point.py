@@ -265,6 +265,7 @@ def _no_less_precise(*args, **kw):
 @pytest.mark.parametrize("D,L,type_op,pot", [
     (4, 8, 0, "harmonic"), (4, 8, 10, "harmonic"),   # one rounding shared by a term
     (2, 13, 1, "none"), (2, 13, 1, "harmonic"), (3, 10, 1, "harmonic"),   # low and high levels in one sum
+    (2, 13, 0, "harmonic"), (2, 13, 10, "harmonic"), (3, 8, 10, "quartic"),   # passes of many inputs
 ])
 def test_smooth_vectors_keep_their_digits(D, L, type_op, pot):
     need_cuda()
