@@ -1578,8 +1578,7 @@ static void plan_work(const evr_sg4_ctx* c, bool fx, int nrhs_v, int smem_double
       const int want = std::min(nrhs_v, rcap);
       r = std::min(want, (int)FX_MAXR);
       const long long fit = std::min<long long>(nbuf, room / ((long long)T.nq * r));
-      slab = std::max(slab, (nbuf - fit) * T.nq * r);
-      if (per > smem_doubles) slab = std::max(slab, per);  // a column left to the FP64 code
+      if (fit < nbuf) slab = std::max(slab, per * r);  // of which columns left to the FP64 code take all
     } else {
       r = (int)std::min<long long>(std::min(nrhs_v, rcap), std::max<long long>(1, smem_doubles / per));
       if (c->nb0 > 1) {  // whole channel groups (both halves of complex columns): 2 nb0 columns
@@ -1777,6 +1776,7 @@ static KParams make_params(evr_sg4_ctx* c, int nrhs_v, int cshift, const double*
   p.geg = c->d_geg;
   p.ed = c->d_ed;
   p.e1 = c->d_e1;
+  p.strict = c->nb_SG == 1 ? 1 : 0;
   return p;
 }
 

@@ -17,10 +17,11 @@
 // bits of each stage's largest value, against the 53 of a double.
 //
 // A right-hand side whose largest entry in a term lies outside 2^+-300 (all
-// subnormal, for instance), or is not finite, and one whose V.x is tiny against
-// max|V| max|x| (a potential so steep that the tails of x carry it), goes
-// through the FP64 item code instead, that column alone.  Operators the scheme
-// does not suit (see fx_prepare in sg4_device.cu) never come here.
+// subnormal, for instance), or is not finite, and one whose result is small
+// against what the scheme's errors could make of it (fx_grid: a potential so
+// steep that the tails of x carry it, say), goes through the FP64 code instead,
+// that column alone.  Operators the scheme does not suit (see fx_prepare in
+// sg4_device.cu) never come here.
 #pragma once
 #include "sg4_items.cuh"
 
@@ -33,7 +34,10 @@ enum {
   FX_FLUSH = 24,                // products |xh ml| <= 2^58 an accumulator takes before it is folded
   FX_TILE = 32,                 // points per tile of the fixed-point metric
   FX_AHEAD = 4,                 // loads ahead of their products from global scratch
-  FX_NONE = -(1 << 30)          // exponent of a type-1 mode without a derivative term
+  FX_NONE = -(1 << 30),         // exponent of a type-1 mode without a derivative term
+  FX_MARGIN_V = 5,              // bits by which a result may stay below its bound (fx_grid)
+  FX_MARGIN_1 = 5,
+  FX_MARGIN_10 = 9
 };
 
 // int2 values of one tile of the fixed-point metric: its D*D elements, rounded
@@ -57,7 +61,7 @@ struct FxShared {
   FxPass ps[FX_MAXD];
   int4 md[FX_MAXD];               // per mode: nq, grid stride, derivative matrix (-1: none), magic of nq
   int moff[FX_MAXD];              // where the mode's matrices start in shared memory
-  unsigned mx[FX_STAGES][FX_MAXR];  // OR of |h| of what stage s stored, per right-hand side
+  unsigned mx[FX_STAGES][FX_MAXR];  // OR of |h| of what stage s stored, per right-hand side (0: see fx_grid)
   int em[FX_MAXR];                // largest biased exponent of the gathered column
   int mv[FX_MAXR];                // largest bits(|h|) + biased exponent of V over the points
   int evmax;                      // largest biased exponent of V
@@ -436,10 +440,25 @@ __device__ __noinline__ void fx_type10_a_dispatch(const KParams& p, const ItemSh
 // V x + sum_i F2_ii (d2_i x) for type 1, V x for type 0 (both into T).  Its
 // exponent bounds both parts: the derivative part from the recorded magnitudes
 // and the row sums, V x from its recorded maximum.
+//
+// x is good to some 2^-57 of its largest value, at every point alike, where an
+// FP64 item keeps 53 bits of each value, so the error of the result is some
+// 2^-57 of max|V| max|x| and of the derivative part's row-sum bound.  An FP64
+// item loses about 2^-53 of the larger part of the result itself.  A column
+// whose result, or V x, stays more than a margin below those bounds is left to
+// the FP64 code: a potential that is large where x is small, derivatives that
+// cancel.  The margins are where errors in units of the FP64 items' reach about
+// one (long-double oracle, columns from N(0, 1) to the lowest function): V x 5
+// bits (4: harmonic vectors on 14 points would go too; 6: twice the error on
+// walls), type 1 5, type 10 9 (its bound takes row sums twice); one less on a
+// basis of a single term, whose FP64 errors no alternating sum adds up.  With
+// the margins 2-D L=13 Morse and wall potentials give 0.4-1.3 times the FP64
+// error (up to 500 times without), at 1 to 2 % of the time of the items.
 template <int C, bool SM>
 __device__ __noinline__ void fx_grid(const KParams& p, const ItemShared& it, FxShared& fs, const FxBufs<C, SM> B) {
   const int D = p.D, nqt = it.nq_t;
   const bool t10 = p.type == 10, hasT = t10 || fs.deriv;
+  const int kD = D > 8 ? 4 : (D > 4 ? 3 : (D > 2 ? 2 : D - 1));
   int a[C], h[C], sP[C];
   unsigned m[C];
 #pragma unroll
@@ -448,7 +467,7 @@ __device__ __noinline__ void fx_grid(const KParams& p, const ItemShared& it, FxS
     // the derivative sum, shifted up by a, has the exponent eT and at most bT bits
     int eT = eX, bT = -100000, aT = 0;
     if (t10) {
-      const int kD = D > 8 ? 4 : (D > 4 ? 3 : (D > 2 ? 2 : D - 1)), aU = fx_head(fs.mx[D + 1][w]);
+      const int aU = fx_head(fs.mx[D + 1][w]);
       aT = max(0, aU - kD);
       eT = eX - aX + p.geg[it.term] - 1 - aT;
       if (fs.mx[D + 1][w]) bT = 59 + max(0, kD - aU) + eT;
@@ -466,9 +485,16 @@ __device__ __noinline__ void fx_grid(const KParams& p, const ItemShared& it, FxS
     h[w] = min(eO - eT, 62);
     sP[w] = 1051 + eO - eX;
     m[w] = 0;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x == blockDim.x - 32) {  // the last warp: idle on a small term
       fs.eo[w] = eO;
-      if (hasV && fs.evmax - 1022 + 59 - aX + eX > eO + 59 + 14) fs.bad |= 1 << w;
+      const int bX = 59 - aX + eX;
+      int need = -100000;
+      if (fs.mx[D][w]) {
+        if (t10) need = bX + kD + p.geg[it.term] - 1 - (FX_MARGIN_10 - p.strict);
+        else if (hasT) need = bT - (FX_MARGIN_1 - p.strict);
+        if (p.V && fs.evmax) need = max(need, hasV ? fs.evmax - 1022 + bX - (FX_MARGIN_V - p.strict) : 100000);
+      }
+      fs.mx[0][w] = (unsigned)(need > bV ? need : -100000);
     }
   }
   const FxArr<C, SM> x = B.x(), O = t10 ? B.x() : B.t();
@@ -546,8 +572,7 @@ __device__ __forceinline__ void fx_body(const KParams& p, const ItemShared& it, 
       const int2 *s1 = p.fxm + it.mo[i][M_BG], *s2 = p.fxm + it.mo[i][p.type == 10 ? M_D1 : M_D2];
       // type 1: the modes' derivative matrices, each kept on its own scale, go
       // into one sum: onto the term's
-      const int sh = fs.deriv && fs.md[i].z >= 0
-                         ? min(p.geg[it.term] - p.e1[i * p.Lp1 + p.terms[it.term].l[i]], 62) : 0;
+      const int sh = fs.md[i].z >= 0 ? it.st[i] : 0;
       for (int e = tid & 31; e < nbq + nqq; e += 32) {
         int2 m = __ldg(e < nbq ? s1 + e : s2 + (e - nbq));
         if (sh > 0 && e >= nbq) m = fx_pack((((((long long)m.x << 29) + m.y) >> (sh - 1)) + 1) >> 1);
@@ -616,13 +641,17 @@ __device__ __forceinline__ void fx_body(const KParams& p, const ItemShared& it, 
   }
   fx_grid<C, SM>(p, it, fs, B);
   __syncthreads();
+  const int lw = tid - ((int)blockDim.x - 32);
+  if (lw >= 0 && lw < C &&
+      (int)fs.mx[0][lw] > (fs.mx[D + 2][lw] ? fs.eo[lw] + 61 - __clz((int)fs.mx[D + 2][lw]) : -90000))
+    atomicOr(&fs.bad, 1 << lw);
   const FxArr<C, SM> O0 = p.type == 10 ? B.x() : B.t(), O1 = p.type == 10 ? B.t() : B.x();
   for (int k = 0; k < D; ++k) {
     const bool last = k == D - 1;
     const int si = !k || fs.ps[D - k].recG ? D + 2 + k : 0;
     fx_pass<C, SM>(p, it, fs, D - 1 - k, false, si, !last && fs.ps[D - 1 - k].recG ? D + 3 + k : 0,
                    (k & 1) ? O1 : O0, (k & 1) ? O0 : O1, last ? 2 : 0);
-    if (!last && si && tid < C) fs.eo[tid] -= fx_head(fs.mx[si][tid]);
+    if (!last && si && lw >= 0 && lw < C) fs.eo[lw] -= fx_head(fs.mx[si][lw]);
     __syncthreads();
   }
 }
@@ -634,68 +663,88 @@ __device__ __forceinline__ double gfx_value(const KParams& p, const ItemShared& 
   return (double)(((long long)g.x << 29) + g.y) * __hiloint2double((1023 + e) << 20, 0);
 }
 
-// One column of an item in FP64 (the exceptional ones), with the operators
-// the fixed-point items take: x in A, then U_1..U_D or O.
-static __device__ __noinline__ void fx_item_fp64(const KParams& p, ItemShared& it, double* A, double* B, int rhs,
+// a matrix row's products with the fibre through a point, added to s in FP64
+__device__ __forceinline__ double fibre_fp64(const double* __restrict__ M, const double* a, int n, int sd, double s) {
+  for (int m = 0; m < n; ++m) s = fma(__ldg(M + m), a[m * sd], s);
+  return s;
+}
+
+// Columns of an item in FP64 (the exceptional ones, r of them from rhs on),
+// with the operators that the fixed-point items take: x in A, then U_1..U_D or
+// O, each column after column.  The sums are those of the FP64 items, in their
+// order (type10_fused, type1_fused).
+static __device__ __noinline__ void fx_item_fp64(const KParams& p, ItemShared& it, double* A, int rhs0, int bad,
                                                  long long tile) {
-  const int D = p.D, nqt = it.nq_t, nbt = it.nb_t;
+  const int r = __popc(bad), rhs = rhs0 + (bad == 2);
+  const int D = p.D, nqt = it.nq_t, nbt = it.nb_t, NQR = nqt * r;
   const long long oq = it.off_nq;
+  double* B = A + NQR;
   if (threadIdx.x == 0) {
     it.rhs0 = rhs;
-    it.r = 1;
+    it.r = r;
   }
   if (threadIdx.x < D) {
-    int rank = 0;
+    int rank = 0, st = 1;
     const int i = threadIdx.x, ni = it.nq[i] - it.nb[i], di = it.nb[i] * it.nq[i];
     for (int j = 0; j < D; ++j) {
       const int kj = (it.nq[j] - it.nb[j]) * di, ki = ni * (it.nb[j] * it.nq[j]);
       rank += j != i && (kj < ki || (kj == ki && j < i));
+      if (j < i) st *= it.nq[j];
     }
     it.ord[rank] = i;
     it.pos[i] = rank;
+    it.st[i] = st;
   }
   double* G0 = (D & 1) ? B : A;
-  for (int k = threadIdx.x; k < nbt; k += blockDim.x) {
-    const int n = __ldg(p.map + it.off_nb + k);
-    G0[k] = n > 0 ? p.psi[vaddr(p, rhs, n - 1, p.ldpsi)] : 0.0;
+  for (int e = threadIdx.x; e < nbt * r; e += blockDim.x) {
+    const int w = e / nbt, n = __ldg(p.map + it.off_nb + e - w * nbt);
+    G0[e] = n > 0 ? p.psi[vaddr(p, rhs + w, n - 1, p.ldpsi)] : 0.0;
   }
   __syncthreads();
   double* x = transform(p, it, true, G0, G0 == A ? B : A);  // == A
-  double* y = x;
+  double* y = p.type == 10 ? x : B;
   if (p.type == 10) {
-    for (int j = 0; j < D; ++j) grid_deriv(p, it, j, M_D1, x, B + (long long)j * nqt, false, 1.0);
-    __syncthreads();
-    for (int q = threadIdx.x; q < nqt; q += blockDim.x) {
+    for (int e = threadIdx.x; e < NQR; e += blockDim.x) {
+      const int q = e % nqt;
       double phi[FX_MAXD];
-      for (int j = 0; j < D; ++j) phi[j] = B[(long long)j * nqt + q];
+      int rem = q;
+      for (int j = 0; j < D; ++j) {
+        const int n = it.nq[j], st = it.st[j], idx = rem % n;
+        rem /= n;
+        phi[j] = fibre_fp64(p.mats + it.mo[j][M_D1] + idx * n, x + e - idx * st, n, st, 0.0);
+      }
       for (int i = 0; i < D; ++i) {
         double u = 0.0;
         for (int j = 0; j < D; ++j)
           u = fma(gfx_value(p, it, __ldg(p.Gfx + fx_g_index(D, tile, q, i * D + j)), i, j), phi[j], u);
-        B[(long long)i * nqt + q] = u;
+        B[(long long)i * NQR + e] = u;
       }
-      x[q] = p.V ? __ldg(p.V + oq + q) * x[q] : 0.0;
     }
     __syncthreads();
-    for (int i = 0; i < D; ++i) {
-      grid_deriv(p, it, i, M_D1, B + (long long)i * nqt, x, true, -0.5);
-      __syncthreads();
-    }
-  } else {
-    y = B;
-    for (int q = threadIdx.x; q < nqt; q += blockDim.x) y[q] = p.V ? __ldg(p.V + oq + q) * x[q] : 0.0;
-    __syncthreads();
-    for (int i = 0; i < D && p.type == 1; ++i) {
-      if (__ldg(p.F2 + i * D + i) != 0.0) grid_deriv(p, it, i, M_D2, x, y, true, __ldg(p.F2 + i * D + i));
-      __syncthreads();
-    }
   }
+  for (int e = threadIdx.x; e < NQR; e += blockDim.x) {
+    const int q = e % nqt;
+    double s = 0.0, o = p.V ? __ldg(p.V + oq + q) * x[e] : 0.0;
+    int rem = q;
+    for (int i = 0; i < D && p.type != 0; ++i) {
+      const int n = it.nq[i], st = it.st[i], idx = rem % n;
+      rem /= n;
+      if (p.type == 10) {
+        s = fibre_fp64(p.mats + it.mo[i][M_D1] + idx * n, B + (long long)i * NQR + e - idx * st, n, st, s);
+      } else if (__ldg(p.F2 + i * D + i) != 0.0) {
+        s = fibre_fp64(p.mats + it.mo[i][M_D2] + idx * n, x + e - idx * st, n, st, 0.0);
+        o = fma(__ldg(p.F2 + i * D + i), s, o);
+      }
+    }
+    y[e] = p.type == 10 ? fma(-0.5, s, o) : o;
+  }
+  __syncthreads();
   const double* yb = transform(p, it, false, y, y == A ? B : A);
   store_contrib(p, it, yb);
 }
 
-// One work item in fixed point (one or two columns), then its
-// exceptional columns, if any, one by one through the FP64 code.
+// One work item in fixed point (one or two columns), then its exceptional
+// columns, if any, through the FP64 code.
 __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, FxShared& fs, int term, int rhs0, int r) {
   const int tid = threadIdx.x, D = p.D;
   if (tid == 0) {
@@ -722,6 +771,9 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
     it.nq[tid] = p.nq_of_l[k];
     it.mg[tid] = it.nq[tid] > 1 ? 0xFFFFFFFFu / (unsigned)it.nq[tid] + 1u : 0u;
     for (int q = 0; q < 4; ++q) it.mo[tid][q] = p.mat_off[k * 8 + 4 * p.transpose + q];
+    // the shift of the mode's type-1 matrix (the FP64 code keeps strides here)
+    const int e1 = p.type == 1 ? __ldg(p.e1 + k) : FX_NONE;
+    it.st[tid] = e1 == FX_NONE ? (p.type == 10 ? 0 : FX_NONE) : min(__ldg(p.geg + term) - e1, 62);
   }
   for (int e = tid; e < FX_STAGES * FX_MAXR; e += blockDim.x) (&fs.mx[0][0])[e] = 0;
   if (tid < FX_MAXR) {
@@ -762,7 +814,7 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
     int md = mo + 2 * di;
     if (i == D - 1) fs.msz = (md + it.nq[i] * it.nq[i] + 1) & ~1;
     if (p.type != 10) {
-      if (p.type == 1 && p.e1[i * p.Lp1 + p.terms[term].l[i]] != FX_NONE) fs.deriv = 1;
+      if (it.st[i] != FX_NONE) fs.deriv = 1;
       else md = -1;
     }
     fs.md[i] = make_int4(it.nq[i], st, md, (int)it.mg[i]);
@@ -805,10 +857,8 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
   }
   if (fs.bad) {
     const int bad = fs.bad;
-    const bool in = (long long)narr * nq <= p.smem_doubles;
-    double* A = in ? reinterpret_cast<double*>(fx_sm) : reinterpret_cast<double*>(slab);
-    for (int j = 0; j < r; ++j)
-      if (bad >> j & 1) fx_item_fp64(p, it, A, A + nq, rhs0 + j, fs.tile);
+    const bool in = (long long)narr * nq * 2 <= p.smem_doubles;
+    fx_item_fp64(p, it, in ? reinterpret_cast<double*>(fx_sm) : reinterpret_cast<double*>(slab), rhs0, bad, fs.tile);
   }
 }
 

@@ -199,6 +199,7 @@ struct KParams {
   long long tbase;           // tile of the first entry (term slices)
   const int* geg;            // [nb_SG] its exponent per term; type 1: that of the term's sum of F2_ii d2GG
   const int* ed;             // [D*Lp1] exponent of d1GG's scale per (mode, level)
+  int strict;                // 1: a basis of one term (fx_grid)
   const int* e1;             // [D*Lp1] type 1: that of F2_ii d2GG's scale, FX_NONE: no such term
 };
 

@@ -270,3 +270,15 @@ def _no_less_precise(*args, **kw):
 def test_smooth_vectors_keep_their_digits(D, L, type_op, pot):
     need_cuda()
     _no_less_precise(D, L, type_op, pot)
+
+
+@pytest.mark.parametrize("D,L,rules,type_op,pot", [
+    (2, 13, (1, 1, 2, 1), 0, "wall"), (2, 13, (1, 1, 2, 1), 1, "wall"), (2, 13, (1, 1, 2, 1), 1, "morse"),
+    (2, 13, (1, 1, 2, 1), 10, "wall"), (3, 10, (1, 1, 2, 1), 1, "wall"), (3, 10, (1, 1, 2, 1), 10, "morse"),
+    (1, 14, (1, 1, 2, 1), 1, "wall"), (1, 14, (1, 1, 2, 1), 10, "morse"),         # a single term
+    (2, 0, (14, 1, 14, 1), 1, "wall"), (2, 0, (14, 1, 14, 1), 10, "morse")])
+def test_potentials_that_the_tails_of_x_carry(D, L, rules, type_op, pot):
+    """V large where x is small: the columns that fixed point would lose digits on go
+    through the FP64 code, one or both of an item's two."""
+    need_cuda()
+    _no_less_precise(D, L, type_op, pot, rules=rules)
