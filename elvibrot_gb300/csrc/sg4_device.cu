@@ -303,8 +303,9 @@ __device__ __forceinline__ int2 fx_from(double g, int k) {
 // The exponent of the fixed-point metric per term (gfx_scan_kernel, one CTA a
 // term): the largest row or column sum of |G_ij| 2^(ed_i + ed_j) over its
 // points is below 2^geg.  bad: a value is not finite, or the points' own sums
-// spread by more than 2^6, which one exponent would not serve; bad[1]: G is not
-// symmetric.
+// spread by more than a factor of two to four, which costs the centre's
+// elements digits (G = exp(0.04 r^2) on 2-D L=13, a factor of 2.3: 1.3 times the
+// FP64 items' error; a factor of 6: 1.9 times); bad[1]: G is not symmetric.
 __global__ void __launch_bounds__(128) gfx_scan_kernel(const TermInfo* terms, int D, int Lp1, const double* G,
                                                        const int* ed, int* geg, int* bad) {
   __shared__ int hi, lo;
@@ -339,7 +340,7 @@ __global__ void __launch_bounds__(128) gfx_scan_kernel(const TermInfo* terms, in
   __syncthreads();
   if (threadIdx.x == 0) {
     geg[blockIdx.x] = hi;
-    if (hi > 150 || hi < -150 || hi - lo > 6) *bad = 1;
+    if (hi > 150 || hi < -150 || hi - lo > 1) *bad = 1;
   }
 }
 
@@ -1193,7 +1194,7 @@ extern "C" int evr_sg4_field_slices(const evr_sg4_ctx* c, long long* nslices) {
 // affine metric.  Fixed point takes one channel, D <= FX_MAXD, types 0, 1 with
 // constant diagonal F2, and 10 with a metric and no volume factors, and fields
 // within 2^+-150; one exponent per term has to serve its metric, so an affine
-// metric may exceed its constant part by at most 2^6 (a metric grid is checked
+// metric may exceed its constant part by at most 4 (a metric grid is checked
 // on the device).  The other operators keep the FP64 items.
 static bool fx_prepare(evr_sg4_ctx* c, const evr_sg4_op_desc* op, bool polyV, bool affG, std::vector<int>& geg) {
   const int D = c->D, Lp1 = c->L + 1;
@@ -1283,7 +1284,7 @@ static bool fx_prepare(evr_sg4_ctx* c, const evr_sg4_op_desc* op, bool polyV, bo
           big = std::max(big, std::max(r, q) * s[i]);
           big0 = std::max(big0, r0 * s[i]);
         }
-        if (!(big > 0x1p-150 && big < 0x1p150 && big <= 64.0 * big0)) return false;
+        if (!(big > 0x1p-150 && big < 0x1p150 && big <= 4.0 * big0)) return false;
         geg[t] = std::ilogb(big) + 1;
       }
     }

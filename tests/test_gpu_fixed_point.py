@@ -282,3 +282,11 @@ def test_potentials_that_the_tails_of_x_carry(D, L, rules, type_op, pot):
     through the FP64 code, one or both of an item's two."""
     need_cuda()
     _no_less_precise(D, L, type_op, pot, rules=rules)
+
+
+@pytest.mark.parametrize("D,L,slope,pot", [(2, 13, 0.12, "harmonic"), (2, 13, 0.04, "harmonic"), (3, 10, 0.12, "none")])
+def test_metrics_that_grow_towards_the_edge(D, L, slope, pot):
+    """G = exp(slope r^2), up to a hundred times its value at the centre: one exponent
+    a term leaves the centre's elements that many fewer bits."""
+    need_cuda()
+    _no_less_precise(D, L, 10, pot, metric=slope)
