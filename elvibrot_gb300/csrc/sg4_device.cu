@@ -2239,14 +2239,16 @@ static void free_multi(evr_sg4_multi* m) {
   delete m;
 }
 
-// one_group: the contexts (of one basis) share a launch, in FP64 unless all run in fixed point.
+// one_group: the contexts (of one basis) share a launch, in FP64 unless all run
+// in fixed point.  fx: a plan made again (multi_refresh), with these contexts in
+// fixed point; of a context that its caller skips nothing is asked.
 static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int flags, bool one_group,
-                        evr_sg4_multi** out) {
+                        evr_sg4_multi** out, const char* fx = nullptr) {
   if (!out) return set_error(EVR_ERR_ARG, "multi_create: NULL output");
   *out = nullptr;
   if (n < 1 || !ctxs || !nrhs) return set_error(EVR_ERR_ARG, "multi_create: NULL argument or n < 1");
   if (flags & ~(EVR_APPLY_TRANSPOSE | EVR_APPLY_COMPLEX)) return set_error(EVR_ERR_ARG, "multi_create: bad flags");
-  for (int k = 0; k < n; ++k) {
+  for (int k = 0; k < n && !fx; ++k) {
     if (!ctxs[k] || !ctxs[k]->have_op) return set_error(EVR_ERR_STATE, "multi_create: context %d has no operator", k);
     if (ctxs[k]->streamed)
       return set_error(EVR_ERR_STATE, "multi_create: context %d streams its operator fields (use evr_sg4_hpsi)", k);
@@ -2268,7 +2270,7 @@ static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int fl
   m->fx.resize(n);
   bool all_fx = true;
   for (int k = 0; k < n; ++k) all_fx = all_fx && ctxs[k]->fx;
-  for (int k = 0; k < n; ++k) m->fx[k] = one_group ? all_fx : ctxs[k]->fx;
+  for (int k = 0; k < n; ++k) m->fx[k] = fx ? fx[k] : (one_group ? all_fx : ctxs[k]->fx);
   // Launch groups, for the fixed-point contexts and for the others.  The
   // contexts with D <= 6 run narrow in a launch of their own when their items
   // fill enough waves and other contexts exist; otherwise one launch takes
@@ -2430,6 +2432,39 @@ extern "C" int evr_sg4_multi_destroy(evr_sg4_multi* m) {
   return EVR_OK;
 }
 
+// The contexts that a call uses (every one without `used`): their operators are
+// of the types and buffer counts that the plan was made for, else an error.  A
+// context may have an operator of the same type that runs in the other
+// arithmetic (a metric that spreads too far for fixed point, say): the plan is
+// then made again in place, which allocates.
+static int multi_refresh(evr_sg4_multi* m, const char* who, const double* const* used) {
+  bool same = true;
+  std::vector<char> fx(m->fx);
+  for (int k = 0; k < m->n; ++k) {
+    evr_sg4_ctx* c = m->ctxs[k];
+    if (used && !used[k]) continue;
+    if (!c->have_op || c->type != m->type[k] || nbuf_for(c) != m->nbuf[k] || c->streamed)
+      return set_error(EVR_ERR_STATE, "%s: the operator of context %d changed since multi_create", who, k);
+    fx[k] = c->fx;
+    same = same && fx[k] == m->fx[k];
+  }
+  if (same) return EVR_OK;
+  std::vector<evr_sg4_ctx*> ctxs;
+  std::vector<int> nrhs;
+  int cshift = 0, transpose = 0;
+  multi_shape(m, &ctxs, &nrhs, &cshift, &transpose);
+  evr_sg4_multi* fresh = nullptr;
+  int rc = multi_create(m->n, ctxs.data(), nrhs.data(),
+                        (cshift ? EVR_APPLY_COMPLEX : 0) | (transpose ? EVR_APPLY_TRANSPOSE : 0), false, &fresh,
+                        fx.data());
+  if (rc) return rc;
+  fresh->type = m->type;  // a skipped context keeps what it was planned for
+  fresh->nbuf = m->nbuf;
+  std::swap(*m, *fresh);
+  free_multi(fresh);  // cudaFree waits for launches that still use the old buffers
+  return EVR_OK;
+}
+
 // One launch group's merged items: the parameters of its contexts (by
 // context) gathered into the group's slots.
 static cudaError_t launch_group(const MGroup& g, const std::vector<KParams>& params, const MItem* items, int n_items,
@@ -2445,13 +2480,12 @@ extern "C" int evr_sg4_multi_hpsi(evr_sg4_multi* m, const double* const* psi, co
                                   void* stream) {
   if (!m || !psi || !hpsi || !ldpsi || !ldh) return set_error(EVR_ERR_ARG, "multi_hpsi: NULL argument");
   cudaStream_t s = (cudaStream_t)stream;
+  if (int rc = multi_refresh(m, "multi_hpsi", psi)) return rc;
   std::vector<KParams> params(m->n);
   int active = 0;
   for (int k = 0; k < m->n; ++k) {
     evr_sg4_ctx* c = m->ctxs[k];
     if (!psi[k]) continue;  // context k is skipped in this call
-    if (!c->have_op || c->type != m->type[k] || nbuf_for(c) != m->nbuf[k] || c->streamed || (m->fx[k] && !c->fx))
-      return set_error(EVR_ERR_STATE, "multi_hpsi: the operator of context %d changed since multi_create", k);
     if (!hpsi[k] || ldpsi[k] < c->nvec || ldh[k] < c->nvec)
       return set_error(EVR_ERR_ARG, "multi_hpsi: bad output or leading dimension for context %d", k);
     const double e0 = E0 ? E0[k] : 0.0, esc = Esc ? Esc[k] : 1.0;
@@ -2508,6 +2542,7 @@ extern "C" int evr_sg4_multi_hpsi(evr_sg4_multi* m, const double* const* psi, co
 // active, so the same bits.
 int evr::multi_bind(evr_sg4_multi* m, int slot, const double* const* psi, double* const* hpsi) {
   if (!m || slot < 0 || slot > 1 || !psi || !hpsi) return set_error(EVR_ERR_ARG, "multi_bind: bad arguments");
+  if (int rc = multi_refresh(m, "multi_bind", nullptr)) return rc;
   std::vector<KParams> params(m->n);
   for (int k = 0; k < m->n; ++k) {
     evr_sg4_ctx* c = m->ctxs[k];

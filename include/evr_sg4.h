@@ -378,7 +378,10 @@ int evr_sg4_cheby_propagate(evr_sg4_ctx* c, const evr_cheby_opts* o, int nrhs, d
  * (EVR_APPLY_COMPLEX, EVR_APPLY_TRANSPOSE); the plan owns the per-call
  * scratch, so the contexts stay usable on their own.  Calling
  * evr_sg4_set_operator with another operator type on a context invalidates
- * the plan (evr_sg4_multi_hpsi returns EVR_ERR_STATE).
+ * the plan (evr_sg4_multi_hpsi returns EVR_ERR_STATE).  An operator of the
+ * same type may run in the other arithmetic (fixed point or FP64): the first
+ * call after that makes the plan again, which allocates and so cannot be
+ * recorded in a CUDA graph.
  * evr_sg4_multi_hpsi: per context k, psi[k] (ld ldpsi[k], device) ->
  * hpsi[k] (ld ldh[k]), scaled by E0[k], Esc[k] (NULL arrays: 0 and 1);
  * psi[k] == NULL skips context k in this call.  A plan is used from one

@@ -12,7 +12,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from elvibrot_gb300 import EVRError, MultiOp, ParamOp, hpsi_multi
+from elvibrot_gb300 import EVRError, MultiOp, ParamOp, SG4Basis, hpsi_multi
 from elvibrot_gb300.configs import make_dipole, make_model
 from oracle.oracle import OracleSG4
 
@@ -338,3 +338,53 @@ def test_multi_chebyshev_graph_replay_is_bit_identical():
     for k in range(3):
         assert torch.equal(outs[0][0][k], outs[1][0][k]), k
         assert np.array_equal(outs[0][1][k], outs[1][1][k]), k
+
+
+def test_plan_follows_an_operator_into_the_other_arithmetic():
+    """set_operator with the same type and buffers, but an operator that fixed point
+    does not take (an off-diagonal F2, a metric that spreads too far), and back: the
+    plan gives each context's own bits, with contexts skipped and in a recorded
+    Chebyshev propagation as well."""
+    need_cuda()
+    rng = np.random.default_rng(77)
+    b3, b2, b4 = (SG4Basis(D, L, scaleQ=np.full(D, 0.5)) for D, L in ((3, 5), (2, 6), (4, 4)))
+    V3, V2 = rng.normal(size=b3.sum_nq), rng.normal(size=b2.sum_nq)
+    mixed = np.triu(rng.normal(size=(3, 3)))
+    G2 = np.exp(rng.uniform(-5.0, 5.0, size=b2.sum_nq * 4))
+    nq = np.prod(b2.tables()[0] + 2, axis=1)
+    one = np.concatenate([np.repeat(np.eye(2).ravel(), n) for n in nq])
+    ops = [ParamOp(b3, 1, V=V3, F2=-0.5 * np.eye(3)), ParamOp(b2, 10, V=V2, G=one),
+           ParamOp(b4, 0, V=rng.normal(size=b4.sum_nq))]
+    nrhs = [2, 3, 1]
+    g = torch.Generator(device="cuda").manual_seed(5)
+    psis = [torch.randn((r, op.basis.N), generator=g, device="cuda", dtype=torch.complex128)
+            for op, r in zip(ops, nrhs)]
+    plan = MultiOp(ops, nrhs, complex_=True)
+
+    def check(skip=None):
+        outs = [torch.zeros_like(p) for p in psis]
+        plan.hpsi([None if k == skip else p for k, p in enumerate(psis)], outs)
+        for k, (op, p) in enumerate(zip(ops, psis)):
+            ref = torch.zeros_like(p)
+            if k != skip:
+                op.hpsi_dev(p, ref)
+            assert torch.equal(outs[k], ref), (k, skip)
+    check()
+    ops[0].set_operator(V=V3, F2=mixed)
+    check()
+    ops[1].set_operator(V=V2, G=G2)
+    check(skip=1)
+    check(skip=0)
+    check()
+    ops[0].set_operator(V=V3, F2=-0.5 * np.eye(3))
+    lo, hi = [-200.0] * 3, [200.0] * 3
+    runs = [[p.clone() for p in psis] for _ in range(2)]
+    plan.cheby_propagate(runs[0], lo, hi, 0.01, 8, 2)
+    for op, p in zip(ops, runs[1]):
+        MultiOp([op], [p.shape[0]], complex_=True).cheby_propagate([p], lo[:1], hi[:1], 0.01, 8, 2)
+    assert all(torch.equal(a, c) for a, c in zip(*runs))
+    check()
+    ops[0].set_operator(V=V3, F2=mixed)
+    plan.cheby_propagate(runs[0], lo, hi, 0.01, 8, 1)
+    MultiOp([ops[0]], [2], complex_=True).cheby_propagate([runs[1][0]], lo[:1], hi[:1], 0.01, 8, 1)
+    assert torch.equal(runs[0][0], runs[1][0])
