@@ -1069,14 +1069,15 @@ extern "C" int evr_sg4_destroy(evr_sg4_ctx* c) {
 }
 
 // V (polynomial) and/or G (affine) on the terms [t0, t1) into the context's
-// field arrays, from index 0.  transpose: the fixed-point metric of a streamed
-// slice for H^T.
+// field arrays, from index 0.  transpose: the fixed-point metric for H^T, of a
+// streamed slice in the place of the forward one.
 static int eval_fields(evr_sg4_ctx* c, long long t0, long long t1, bool V, bool G, cudaStream_t s,
                        bool transpose = false) {
   if (t1 <= t0) return EVR_OK;
+  int2* Gfx = transpose && c->d_GfxT ? c->d_GfxT : c->d_Gfx;
   const long long g0 = c->terms[t0].off_nq, g1 = t1 < c->nb_SG ? c->terms[t1].off_nq : c->z.sum_nq;
   const bool split = c->d_units != nullptr;  // one channel: V and the fixed-point metric
-  if (split && (V || (G && c->d_Gfx))) {
+  if (split && (V || (G && Gfx))) {
     FieldArgs a = {};
     a.units = c->d_units + c->unit_start[t0];
     a.terms = c->d_terms;
@@ -1091,7 +1092,7 @@ static int eval_fields(evr_sg4_ctx* c, long long t0, long long t1, bool V, bool 
     a.gp0 = g0;
     a.G0 = c->d_G0;
     a.G1 = c->d_G1;
-    a.Gfx = G ? c->d_Gfx : nullptr;
+    a.Gfx = G ? Gfx : nullptr;
     a.geg = c->d_geg;
     a.ed = c->d_ed;
     a.fxterms = c->d_fxterms;
@@ -1294,7 +1295,7 @@ static bool fx_prepare(evr_sg4_ctx* c, const evr_sg4_op_desc* op, bool polyV, bo
 
 // The fixed-point grid of a resident metric G (c->d_G on the device; affine:
 // evaluated into d_Gfx with the double one), and its transpose if G is not
-// symmetric.  Without memory for them, or with a metric that one exponent per
+// symmetric (affine: evaluated as well, so that a streamed slice has its bits).  Without memory for them, or with a metric that one exponent per
 // term does not serve, the operator stays with the FP64 items.
 static int fx_metric(evr_sg4_ctx* c, bool affine) {
   const int D = c->D;
@@ -1324,9 +1325,12 @@ static int fx_metric(evr_sg4_ctx* c, bool affine) {
   if (!affine)
     gfx_convert_kernel<<<(unsigned)c->nb_SG, 256>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg,
                                                   c->d_fxterms, c->d_Gfx, 0);
-  if (flags[1])
+  if (flags[1] && affine) {
+    if (int rc = eval_fields(c, 0, c->nb_SG, false, true, 0, true)) return rc;
+  } else if (flags[1]) {
     gfx_convert_kernel<<<(unsigned)c->nb_SG, 256>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg,
                                                   c->d_fxterms, c->d_GfxT, 1);
+  }
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaDeviceSynchronize());
   return EVR_OK;

@@ -235,7 +235,7 @@ int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi, long long 
  * as the reference builds them term by term inside its term loop when they
  * are not kept in memory (get_OpGrid_type10_OF_ONEDP_FOR_SG4,
  * SRC/sub_Operator/sub_OpPsi_SG4.f90:2536, called at :1553).  The per-term
- * contributions and their ordered accumulation are unchanged, so results are
+ * contributions and their accumulation are unchanged, so results are
  * bit-identical to resident fields.  Grids passed as arrays are always
  * resident.  0 (the default): resident.  evr_sg4_hpsi/_cplx/_apply (not
  * _plain) and everything built on them accept streamed contexts; the

@@ -11,7 +11,7 @@ import pytest
 
 torch = pytest.importorskip("torch")
 
-from elvibrot_gb300 import EVRError, MultiOp
+from elvibrot_gb300 import EVRError, MultiOp, ParamOp, SG4Basis
 from elvibrot_gb300.configs import make_model
 
 from oracle.oracle import OracleSG4
@@ -107,3 +107,23 @@ def test_streamed_rejections():
         st.hpsi_dev(P, torch.empty_like(P), plain=True)
     with pytest.raises(EVRError):
         MultiOp([st], [2])
+
+
+@pytest.mark.parametrize("D,L", [(3, 7), (5, 5)])
+def test_streamed_metric_that_is_not_symmetric(D, L):
+    """H and H^T of an affine metric that is not symmetric: streamed slices give the bits
+    of the resident fields in both directions."""
+    need_cuda()
+    b = SG4Basis(D, L, scaleQ=np.full(D, 0.5))
+    rng = np.random.default_rng(D)
+    kw = dict(G0=np.eye(D) + 0.1 * rng.normal(size=(D, D)), G1=0.01 * rng.normal(size=(D, D, D)))
+    res = ParamOp(b, 10, **kw)
+    st = ParamOp(b, 10, field_budget=b.sum_nq * 8 * D * D // 4, **kw)
+    assert res.field_slices == 0 and st.field_slices >= 4
+    P = _rand(b.N, 3, False, 6)
+    for transpose in (False, True):
+        x, y = torch.empty_like(P), torch.empty_like(P)
+        res.hpsi_dev(P, x, transpose=transpose)
+        st.hpsi_dev(P, y, transpose=transpose)
+        torch.cuda.synchronize()
+        assert torch.equal(x, y), transpose
