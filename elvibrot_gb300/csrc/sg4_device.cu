@@ -1293,28 +1293,28 @@ static bool fx_prepare(evr_sg4_ctx* c, const evr_sg4_op_desc* op, bool polyV, bo
   return true;
 }
 
-// The fixed-point grid of a resident metric G (c->d_G on the device; affine:
-// evaluated into d_Gfx with the double one), and its transpose if G is not
-// symmetric (affine: evaluated as well, so that a streamed slice has its bits).  Without memory for them, or with a metric that one exponent per
-// term does not serve, the operator stays with the FP64 items.
-static int fx_metric(evr_sg4_ctx* c, bool affine) {
+// The fixed-point grid of a metric grid (c->d_G on the device), and its
+// transpose if G is not symmetric.  With a metric that one exponent per term
+// does not serve, or where the copies would take more than half of the memory
+// that is free, the operator stays with the FP64 items.
+static int fx_metric(evr_sg4_ctx* c) {
   const int D = c->D;
-  const size_t bytes = (size_t)c->slice_tiles * fx_tile_size(D) * sizeof(int2);
-  int flags[2] = {0, affine && !c->G_sym};
-  if (!affine) {
-    int* d_flags = nullptr;
-    CUDA_TRY(cudaMemcpy(c->d_terms, c->terms.data(), c->terms.size() * sizeof(TermInfo), cudaMemcpyHostToDevice));
-    int rc = upload(&d_flags, flags, 2);
-    if (!rc) rc = upload<int>(&c->d_geg, nullptr, c->terms.size());
-    if (!rc) {
-      gfx_scan_kernel<<<(unsigned)c->nb_SG, 128>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg, d_flags);
-      if (cudaMemcpy(flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost) != cudaSuccess)
-        rc = set_error(EVR_ERR_CUDA, "set_operator: metric scan: %s", cudaGetErrorString(cudaGetLastError()));
-    }
-    if (d_flags) cudaFree(d_flags);
-    if (rc) return rc;
+  const size_t bytes = (size_t)c->all_tiles * fx_tile_size(D) * sizeof(int2);
+  int flags[2] = {0, 0};
+  int* d_flags = nullptr;
+  CUDA_TRY(cudaMemcpy(c->d_terms, c->terms.data(), c->terms.size() * sizeof(TermInfo), cudaMemcpyHostToDevice));
+  int rc = upload(&d_flags, flags, 2);
+  if (!rc) rc = upload<int>(&c->d_geg, nullptr, c->terms.size());
+  if (!rc) {
+    gfx_scan_kernel<<<(unsigned)c->nb_SG, 128>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg, d_flags);
+    if (cudaMemcpy(flags, d_flags, sizeof(flags), cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = set_error(EVR_ERR_CUDA, "set_operator: metric scan: %s", cudaGetErrorString(cudaGetLastError()));
   }
-  if (flags[0] || (!affine && cudaMalloc(&c->d_Gfx, bytes) != cudaSuccess) ||
+  if (d_flags) cudaFree(d_flags);
+  if (rc) return rc;
+  size_t avail = 0, total = 0;
+  CUDA_TRY(cudaMemGetInfo(&avail, &total));
+  if (flags[0] || (flags[1] ? 2 : 1) * bytes > avail / 2 || cudaMalloc(&c->d_Gfx, bytes) != cudaSuccess ||
       (flags[1] && cudaMalloc(&c->d_GfxT, bytes) != cudaSuccess)) {
     cudaGetLastError();
     if (c->d_Gfx) cudaFree(c->d_Gfx);
@@ -1322,15 +1322,27 @@ static int fx_metric(evr_sg4_ctx* c, bool affine) {
     c->fx = false;
     return EVR_OK;
   }
-  if (!affine)
+  for (int t = 0; t < 1 + flags[1]; ++t)
     gfx_convert_kernel<<<(unsigned)c->nb_SG, 256>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg,
-                                                  c->d_fxterms, c->d_Gfx, 0);
-  if (flags[1] && affine) {
-    if (int rc = eval_fields(c, 0, c->nb_SG, false, true, 0, true)) return rc;
-  } else if (flags[1]) {
-    gfx_convert_kernel<<<(unsigned)c->nb_SG, 256>>>(c->d_terms, D, c->L + 1, c->d_G, c->d_ed, c->d_geg,
-                                                  c->d_fxterms, c->d_GfxT, 1);
+                                                  c->d_fxterms, t ? c->d_GfxT : c->d_Gfx, t);
+  CUDA_TRY(cudaGetLastError());
+  CUDA_TRY(cudaDeviceSynchronize());
+  return EVR_OK;
+}
+
+// The resident affine metric in double, for what reads it beside the
+// fixed-point items: the FP64 items of a mixed pair, the diagonal.
+static int need_G(evr_sg4_ctx* c) {
+  if (!c->has_G || c->d_G || c->streamed) return EVR_OK;
+  if (cudaMalloc(&c->d_G, (size_t)c->z.sum_nq * c->D * c->D * 8) != cudaSuccess) {
+    cudaGetLastError();
+    c->d_G = nullptr;
+    return set_error(EVR_ERR_ALLOC, "no memory for the metric in double (%lld points)", c->z.sum_nq);
   }
+  const long long blocks = std::max<long long>(1, std::min<long long>((c->z.sum_nq + 255) / 256, 8LL * c->num_sms));
+  fields_kernel<<<(unsigned)blocks, 256>>>(c->d_terms, c->nb_SG, c->d_pt_start, c->d_nq_of_l, c->d_x, c->d_x_off, c->D,
+                                           c->L + 1, 0, nullptr, nullptr, nullptr, c->d_G0, c->d_G1, c->d_G, 0,
+                                           c->z.sum_nq, c->nb0, c->z.sum_nq, c->G_sym);
   CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaDeviceSynchronize());
   return EVR_OK;
@@ -1391,30 +1403,71 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       }
     }
   }
-  // fields given in analytic form are streamed per term slice when they exceed the budget
+  memset(c->F2, 0, sizeof(c->F2));
+  memset(c->F1, 0, sizeof(c->F1));
+  if (op->type == 1) {
+    if (op->F2)
+      for (int i = 0; i < D; ++i)
+        for (int j = i; j < D; ++j) c->F2[i * D + j] = op->F2[i * D + j];
+    if (op->F1)
+      for (int i = 0; i < D; ++i) c->F1[i] = op->F1[i];
+  }
+  c->has_G = op->type == 10 && (op->G_grid || affG);
+  c->G_sym = 0;
+  if (affG) {
+    bool sym = true;
+    for (int i = 0; i < D && sym; ++i)
+      for (int j = 0; j < D && sym; ++j) {
+        if (op->G0 && memcmp(&op->G0[i * D + j], &op->G0[j * D + i], sizeof(double)) != 0) sym = false;
+        for (int k = 0; k < D && sym && op->G1; ++k)
+          if (memcmp(&op->G1[((size_t)i * D + j) * D + k], &op->G1[((size_t)j * D + i) * D + k], sizeof(double)))
+            sym = false;
+      }
+    c->G_sym = sym ? 1 : 0;
+  }
+  std::vector<int> geg;
+  bool fx = fx_prepare(c, op, polyV, affG, geg);
+  // Fields given in analytic form are streamed per term slice when in double
+  // they exceed the budget.  The fixed-point metric takes whole tiles of 32
+  // points (and, resident and not symmetric, its transpose): where it would
+  // exceed the budget and the double one does not, the FP64 items keep the
+  // operator, resident or streamed.
   const bool grids = op->V_grid || (op->type == 10 && (op->G_grid || op->Jac_grid || op->sqRho_grid)) ||
                      (op->type == 1 && (op->F2_grid || op->F1_grid));
   const double bpp = 8.0 * (polyV ? 1 : 0) + 8.0 * D * D * (affG ? 1 : 0);  // bytes per grid point
   const bool stream = c->field_budget > 0 && !grids && (polyV || affG) && bpp * (double)snq > (double)c->field_budget;
   if (stream && c->nb0 > 1)
     return set_error(EVR_ERR_ARG, "field budget: streamed fields take one channel (nb0 = %d)", c->nb0);
+  auto tiles_of = [](long long q) { return (q + FX_TILE - 1) / FX_TILE; };
+  const double tile_bytes = (double)fx_tile_size(D) * sizeof(int2), vpt = polyV ? 8.0 : 0.0;
+  if (fx && affG && c->field_budget > 0 && !grids) {
+    if (stream) {
+      for (long long t = 0; t < c->nb_SG && fx; ++t)
+        fx = vpt * c->terms[t].nq + tile_bytes * tiles_of(c->terms[t].nq) <= (double)c->field_budget;
+    } else {
+      fx = vpt * snq + tile_bytes * c->all_tiles * (c->G_sym ? 1 : 2) <= (double)c->field_budget;
+    }
+  }
   long long slice_pts = snq, slice_tiles = c->all_tiles;
   if (stream) {
-    const long long cap = (long long)((double)c->field_budget / bpp);
     c->slice_term.push_back(0);
+    double bytes = 0.0;
     long long pts = 0, tiles = 0;
     slice_pts = slice_tiles = 0;
     for (long long t = 0; t < c->nb_SG; ++t) {
       const long long q = c->terms[t].nq;
-      if (q > cap)
+      const double b = fx && affG ? vpt * q + tile_bytes * tiles_of(q) : bpp * q;
+      if (b > (double)c->field_budget)
         return set_error(EVR_ERR_ARG, "field budget %lld B is below the fields of term %lld (%lld points)",
                          c->field_budget, t, q);
-      if (pts + q > cap) {
+      if (bytes + b > (double)c->field_budget) {
         c->slice_term.push_back(t);
+        bytes = 0.0;
         pts = tiles = 0;
       }
+      bytes += b;
       pts += q;
-      tiles += (q + FX_TILE - 1) / FX_TILE;
+      tiles += tiles_of(q);
       slice_pts = std::max(slice_pts, pts);
       slice_tiles = std::max(slice_tiles, tiles);
     }
@@ -1425,32 +1478,23 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
       if (!std::isfinite(op->V_grid[k])) return set_error(EVR_ERR_NUMERIC, "V_grid[%lld] is not finite", k);
     if ((rc = upload(&c->d_V, op->V_grid, (size_t)nvg))) return rc;
   }
-  memset(c->F2, 0, sizeof(c->F2));
-  memset(c->F1, 0, sizeof(c->F1));
-  if (op->type == 1) {
-    if (op->F2)
-      for (int i = 0; i < D; ++i)
-        for (int j = i; j < D; ++j) c->F2[i * D + j] = op->F2[i * D + j];
-    if (op->F1)
-      for (int i = 0; i < D; ++i) c->F1[i] = op->F1[i];
-  }
-  std::vector<int> geg;
-  c->has_G = op->type == 10 && (op->G_grid || affG);
-  bool fx = fx_prepare(c, op, polyV, affG, geg);
   if (fx && !geg.empty() && (rc = upload(&c->d_geg, geg.data(), geg.size()))) return rc;
   if (polyV) CUDA_TRY(cudaMalloc(&c->d_V, (size_t)slice_pts * 8 * c->nb0 * c->nb0));
   if (op->type == 10) {
     if (op->G_grid) {
       if ((rc = upload(&c->d_G, op->G_grid, (size_t)snq * D * D))) return rc;
     } else if (affG) {
-      // streamed: the metric in the form that the items read; resident: in both
-      if (!fx || !stream) CUDA_TRY(cudaMalloc(&c->d_G, (size_t)slice_pts * D * D * 8));
-      if (fx && cudaMalloc(&c->d_Gfx, (size_t)slice_tiles * fx_tile_size(D) * sizeof(int2)) != cudaSuccess) {
+      // in the form that the items read (need_G forms the double one where it is asked for)
+      const size_t bytes = (size_t)slice_tiles * fx_tile_size(D) * sizeof(int2);
+      if (fx && (cudaMalloc(&c->d_Gfx, bytes) != cudaSuccess ||
+                 (!stream && !c->G_sym && cudaMalloc(&c->d_GfxT, bytes) != cudaSuccess))) {
         cudaGetLastError();
+        if (c->d_Gfx) cudaFree(c->d_Gfx);
         c->d_Gfx = nullptr;
         if (stream) return set_error(EVR_ERR_ALLOC, "set_operator: no memory for a slice of the metric");
         fx = false;
       }
+      if (!fx) CUDA_TRY(cudaMalloc(&c->d_G, (size_t)slice_pts * D * D * 8));
     }
     if (op->Jac_grid) {
       for (long long k = 0; k < snq; ++k)
@@ -1530,29 +1574,18 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
                   (rc = upload(&c->d_Vfac, vfac.data(), vfac.size()))))
       return rc;
     c->V_nterms = polyV ? op->V_nterms : 0;
-    c->G_sym = 0;
-    if (affG) {
-      bool sym = true;
-      for (int i = 0; i < D && sym; ++i)
-        for (int j = 0; j < D && sym; ++j) {
-          if (op->G0 && memcmp(&op->G0[i * D + j], &op->G0[j * D + i], sizeof(double)) != 0) sym = false;
-          for (int k = 0; k < D && sym && op->G1; ++k)
-            if (memcmp(&op->G1[((size_t)i * D + j) * D + k], &op->G1[((size_t)j * D + i) * D + k], sizeof(double)))
-              sym = false;
-        }
-      c->G_sym = sym ? 1 : 0;
-    }
     if (affG && op->G0 && (rc = upload(&c->d_G0, op->G0, (size_t)D * D))) return rc;
     if (affG && op->G1 && (rc = upload(&c->d_G1, op->G1, (size_t)D * D * D))) return rc;
     if (c->nb0 == 1 && (polyV || (affG && fx)) && (rc = split_fields(c, op, vfac, polyV))) return rc;
     if (!stream) {
       if ((rc = eval_fields(c, 0, c->nb_SG, polyV, affG, 0))) return rc;
+      if (c->d_GfxT && (rc = eval_fields(c, 0, c->nb_SG, false, true, 0, true))) return rc;
       CUDA_TRY(cudaDeviceSynchronize());
     }
   }
   c->fx = fx;
   c->slice_tiles = slice_tiles;
-  if (fx && op->type == 10 && !stream && (rc = fx_metric(c, op->G_grid == nullptr))) return rc;
+  if (fx && op->G_grid && (rc = fx_metric(c))) return rc;
   if (c->fx && !c->d_GfxT) c->d_GfxT = c->d_Gfx;  // streamed: the slice is evaluated for the direction asked for
   c->streamed = stream;
   c->have_op = true;
@@ -2274,7 +2307,11 @@ static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int fl
   m->fx.resize(n);
   bool all_fx = true;
   for (int k = 0; k < n; ++k) all_fx = all_fx && ctxs[k]->fx;
-  for (int k = 0; k < n; ++k) m->fx[k] = fx ? fx[k] : (one_group ? all_fx : ctxs[k]->fx);
+  for (int k = 0; k < n; ++k) {
+    m->fx[k] = fx ? fx[k] : (one_group ? all_fx : ctxs[k]->fx);
+    if (one_group && !m->fx[k])
+      if (int rc = need_G(ctxs[k])) return fail(rc);
+  }
   // Launch groups, for the fixed-point contexts and for the others.  The
   // contexts with D <= 6 run narrow in a launch of their own when their items
   // fill enough waves and other contexts exist; otherwise one launch takes
@@ -2916,6 +2953,17 @@ extern "C" int evr_sg4_diagonal(evr_sg4_ctx* c, double* diag, void* stream) {
   if (!c->have_op) return set_error(EVR_ERR_STATE, "diagonal: set_operator was not called");
   if (c->nb0 > 1 || c->streamed || c->d_Jac || c->d_sqRho || c->n_t1 > 0)
     return evr_sg4_diagonal_by_apply(c, diag, stream);
+  const bool temp = c->has_G && !c->d_G;  // the metric in double, for this call
+  if (need_G(c) != EVR_OK) return evr_sg4_diagonal_by_apply(c, diag, stream);
+  struct Guard {
+    evr_sg4_ctx* c;
+    bool on;
+    ~Guard() {
+      if (!on) return;
+      cudaFree(c->d_G);  // waits for the kernel
+      c->d_G = nullptr;
+    }
+  } guard{c, temp && c->d_G};
   cudaStream_t s = (cudaStream_t)stream;
   const int D = c->D;
   std::vector<DiagPat> pats;

@@ -236,7 +236,10 @@ int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi, long long 
  * are not kept in memory (get_OpGrid_type10_OF_ONEDP_FOR_SG4,
  * SRC/sub_Operator/sub_OpPsi_SG4.f90:2536, called at :1553).  The per-term
  * contributions and their accumulation are unchanged, so results are
- * bit-identical to resident fields.  Grids passed as arrays are always
+ * bit-identical to resident fields.  (In fixed point a metric takes whole
+ * tiles of 32 points.  Where those do not fit the budget -- one term's when
+ * streamed, all terms' when resident -- and the metric in double does, the FP64
+ * items keep the operator, and the two differ in rounding.)  Grids passed as arrays are always
  * resident.  0 (the default): resident.  evr_sg4_hpsi/_cplx/_apply (not
  * _plain) and everything built on them accept streamed contexts; the
  * per-term path, the multi-context plans and evr_sg4_hpsi_noalloc return

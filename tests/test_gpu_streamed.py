@@ -127,3 +127,92 @@ def test_streamed_metric_that_is_not_symmetric(D, L):
         st.hpsi_dev(P, y, transpose=transpose)
         torch.cuda.synchronize()
         assert torch.equal(x, y), transpose
+
+
+def _held(make):
+    """(operator, device bytes that making it took)"""
+    import gc
+    gc.collect()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    op = make()
+    torch.cuda.synchronize()
+    return op, free - torch.cuda.mem_get_info()[0]
+
+
+def test_resident_metric_is_held_once_and_within_the_budget():
+    """A resident affine metric takes what its double values would (tiles of 32 points,
+    an even number of elements), beside the rest of the context; a budget that the
+    double metric fits, and the fixed-point one does not, holds; the diagonal forms the
+    double metric for its own time."""
+    need_cuda()
+    m = make_model(6, 7, 10, 20261219)
+    b = m.basis()
+    fields = b.sum_nq * 8 * 37
+    base = _held(lambda: ParamOp(b, 0, V_poly=m.V))[1]  # the context and V
+    op, held = _held(lambda: m.operator(basis=b))
+    assert held - base <= 1.15 * fields + (8 << 20)
+    before = torch.cuda.mem_get_info()[0]
+    d = op.diagonal()
+    torch.cuda.synchronize()
+    assert before - torch.cuda.mem_get_info()[0] <= (8 << 20)
+    ref = op.diagonal(by_apply=True)
+    assert float((d - ref).abs().max() / ref.abs().max()) <= 1e-12
+    # not symmetric: two fixed-point copies do not fit, the double metric does
+    rng = np.random.default_rng(3)
+    kw = dict(G0=np.eye(6) + 0.01 * rng.normal(size=(6, 6)), G1=0.01 * rng.normal(size=(6, 6, 6)))
+    tight, held = _held(lambda: ParamOp(b, 10, field_budget=int(1.3 * fields), **kw))
+    assert tight.field_slices == 0 and held - base <= 1.3 * fields + (8 << 20)
+    free = ParamOp(b, 10, **kw)
+    P = _rand(b.N, 2, False, 9)
+    x, y = torch.empty_like(P), torch.empty_like(P)
+    for transpose in (False, True):
+        tight.hpsi_dev(P, x, transpose=transpose)
+        free.hpsi_dev(P, y, transpose=transpose)
+        torch.cuda.synchronize()
+        assert float((x - y).abs().max() / y.abs().max()) <= 1e-12
+
+
+def test_slices_hold_the_padded_metric_within_the_budget():
+    """Slices are cut by what their fixed-point metric takes; a budget that the largest
+    term only fits in double still streams, in FP64."""
+    need_cuda()
+    m = make_model(3, 8, 10, 20261220)
+    b = m.basis()
+    nq = np.prod(b.tables()[0] + 2, axis=1)
+    padded = 8 * nq + 8 * 320 * (-(-nq // 32))  # V, and tiles of 32 points of 10 elements
+    P = _rand(b.N, 3, False, 2)
+    ref, out = torch.empty_like(P), torch.empty_like(P)
+    m.operator(basis=b).hpsi_dev(P, ref)
+    for budget, exact in ((int(padded.max()), True), (int(padded.max()) - 1, False), (int(nq.max()) * 80, False)):
+        st = m.operator(basis=b, field_budget=budget)
+        slices, used = 1, 0
+        for p, q in zip(padded if exact else 80 * nq, nq):
+            if used + p > budget:
+                slices, used = slices + 1, 0
+            used += p
+        assert st.field_slices == slices
+        st.hpsi_dev(P, out)
+        torch.cuda.synchronize()
+        assert torch.equal(out, ref) if exact else float((out - ref).abs().max() / ref.abs().max()) <= 1e-12
+
+
+def test_pair_of_operators_in_different_arithmetics():
+    """H0 with an affine metric (fixed point on its own) and a dipole that only FP64
+    takes, scaled out of the fixed-point range: the pair runs in FP64 on the double
+    metric, and agrees with the pair of the unscaled dipole."""
+    need_cuda()
+    from elvibrot_gb300.configs import make_dipole
+    m = make_model(3, 5, 10, 20261221)
+    b = m.basis()
+    H0, mu = m.operator(basis=b), ParamOp(b, 0, V_poly=make_dipole(m, 4))
+    big = make_dipole(m, 4)
+    big.coef = big.coef * 2.0 ** 200
+    E = np.random.default_rng(1).normal(0.0, 1e-2, 6)
+    P = _rand(b.N, 1, True, 3)[0]
+    P = (P / P.norm()).contiguous()
+    a, c = P.clone(), P.clone()
+    H0.rk4_field(mu, E, a, 2.0, nsub=4)
+    H0.rk4_field(ParamOp(b, 0, V_poly=big), E * 2.0 ** -200, c, 2.0, nsub=4)
+    torch.cuda.synchronize()
+    assert float((a - c).norm()) <= 1e-11
