@@ -857,7 +857,7 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
   }
   if (fs.bad) {
     const int bad = fs.bad;
-    const bool in = (long long)narr * nq * 2 <= p.smem_doubles;
+    const bool in = (long long)narr * NQR <= p.smem_doubles;  // else the plan has a slab for this item's arrays
     fx_item_fp64(p, it, in ? reinterpret_cast<double*>(fx_sm) : reinterpret_cast<double*>(slab), rhs0, bad, fs.tile);
   }
 }

@@ -290,3 +290,24 @@ def test_metrics_that_grow_towards_the_edge(D, L, slope, pot):
     a term leaves the centre's elements that many fewer bits."""
     need_cuda()
     _no_less_precise(D, L, 10, pot, metric=slope)
+
+
+@pytest.mark.parametrize("nrhs", [1, 2, 3])
+@pytest.mark.parametrize("nb,nq", [(3, 4), (4, 5), (5, 6)])
+def test_exceptional_columns_of_terms_around_the_shared_memory(nb, nq, nrhs):
+    """A term whose arrays fit a CTA's shared memory twice, once, or not at all (4-D type
+    10: 5 nq^4 values of 3776), with a column that the FP64 code takes, alone or as one
+    or both of a pair."""
+    need_cuda()
+    b = SG4Basis(4, 0, A_nb=nb, A_nq=nq, scaleQ=np.full(4, 0.5))
+    V = np.random.default_rng(nq).normal(size=b.sum_nq)
+    op = ParamOp(b, 10, V=V, G0=np.eye(4), G1=np.zeros((4, 4, 4)))
+    psi = random_psi(b.N, nrhs, 17)
+    ref = gpu_apply(op, psi)
+    for far in ([0], [nrhs - 1], list(range(nrhs))):
+        x = psi.copy()
+        x[:, far] = np.ldexp(x[:, far], 700)
+        got = gpu_apply(op, x)
+        near = [j for j in range(nrhs) if j not in far]
+        assert np.array_equal(got[:, near], ref[:, near])
+        assert rel_err(np.ldexp(got[:, far], -700), ref[:, far]) <= TOL
