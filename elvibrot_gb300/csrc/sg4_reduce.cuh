@@ -1,15 +1,17 @@
 // sg4_reduce.cuh -- the weighted accumulation of the Smolyak terms
 // (tabR_AT_iG_TO_tabPackedBasis, sub_module_basis_BtoG_GtoB_SG4.f90:1255):
-// the sum of a packed function's term contributions, exact before its one
-// rounding.
+// the sum of a packed function's term contributions.
 //
 // The Smolyak weights alternate in sign and cancel, so plain sums lose digits,
 // and compensated ones run seven dependent FP64 additions a value on a unit
 // that does two a clock and SM.  Here the values of a function and column are
 // added as 128-bit integers on the scale of their largest exponent: integer
 // instructions only, and an associative sum, so that a block's threads share
-// it freely and the result does not depend on how.  Bound by the latency of an
-// index and a value load.  Against two kernels of compensated chunk sums and
+// it freely and the result does not depend on how.  A value is cut below
+// 2^-116 of the largest one's leading bit (2^(k-116) for a list of up to
+// 2^(9+k) values), so n values are summed to n 2^-116 of it, against some
+// n 2^-106 for the compensated sums, and rounded once.  Bound by the latency of
+// an index and a value load.  Against two kernels of compensated chunk sums and
 // joins: 4-D L=7, one complex vector, an order-30 Chebyshev step 1.53 -> 1.01 ms
 // and an RK4 stage's two kernels 33 -> 10 us; one vector of a 3-D L=6 operator
 // 34.5 -> 24.3 us.
@@ -21,18 +23,20 @@ namespace evr {
 #define EVR_SUM_THREADS 128
 #define EVR_SUM_KEEP 4  // values a thread keeps between the two passes
 
-// the largest value's 53-bit mantissa has its top at bit 96: 30 bits above for
-// the number of values, and the sign; 44 bits below its last
-__device__ __forceinline__ __int128 sum_term(double x, int emax) {
+// the largest value's 53-bit mantissa has its top at bit 116 - k: above are the
+// sign and room for 2^(9+k) values
+__device__ __forceinline__ int sum_shift(long long n) { return n > 512 ? 55 - __clzll(n - 1) : 0; }
+
+__device__ __forceinline__ __int128 sum_term(double x, int emax, int k) {
   const long long b = __double_as_longlong(x);
   const int e = (int)(b >> 52) & 0x7ff;
   const unsigned long long m = ((unsigned long long)b & 0xFFFFFFFFFFFFFull) | (e ? 0x10000000000000ull : 0ull);
-  const int d = min(emax - max(e, 1), 127);
-  const __int128 v = (__int128)(((unsigned __int128)m << 44) >> d);
+  const int d = min(emax - max(e, 1) + k, 127);
+  const __int128 v = (__int128)(((unsigned __int128)m << 64) >> d);
   return b < 0 ? -v : v;
 }
 
-__device__ __forceinline__ double sum_value(__int128 v, int emax) {
+__device__ __forceinline__ double sum_value(__int128 v, int emax, int k) {
   const bool neg = v < 0;
   unsigned __int128 a = neg ? (unsigned __int128)(-v) : (unsigned __int128)v;
   if (a == 0) return 0.0;
@@ -40,7 +44,7 @@ __device__ __forceinline__ double sum_value(__int128 v, int emax) {
   const int lz = hi ? __clzll((long long)hi) : 64 + __clzll((long long)(unsigned long long)a);
   a <<= lz;
   const unsigned long long top = (unsigned long long)(a >> 64) | ((unsigned long long)a != 0);  // sticky
-  const double r = scalbn(__ull2double_rn(top), 64 - lz + emax - 1075 - 44);
+  const double r = scalbn(__ull2double_rn(top), k - lz + emax - 1075);
   return neg ? -r : r;
 }
 
@@ -64,6 +68,7 @@ __device__ __forceinline__ void sum_function(const double* __restrict__ contrib,
   const int step = EVR_SUM_THREADS / cw;
   const int v = v0 + col;
   const bool on = v < nv;
+  const int k2 = sum_shift(q1 - q0);
   double keep[EVR_SUM_KEEP];
   int em = 1;
   const long long qs = q0 + tid / cw;
@@ -87,10 +92,10 @@ __device__ __forceinline__ void sum_function(const double* __restrict__ contrib,
   __int128 s = 0;
   if (on) {
 #pragma unroll
-    for (int k = 0; k < EVR_SUM_KEEP; ++k) s += sum_term(keep[k], em);
+    for (int k = 0; k < EVR_SUM_KEEP; ++k) s += sum_term(keep[k], em, k2);
 #pragma unroll 4
     for (long long q = qs + (long long)EVR_SUM_KEEP * step; q < q1; q += step)
-      s += sum_term(contrib[idx[q] * nv + v], em);
+      s += sum_term(contrib[idx[q] * nv + v], em, k2);
   }
   for (int off = 16; off >= cw; off >>= 1) s += shfl_xor128(s, off);
   if (lane < cw) ss[warp * cw + lane] = s;
@@ -99,7 +104,7 @@ __device__ __forceinline__ void sum_function(const double* __restrict__ contrib,
     s = 0;
 #pragma unroll
     for (int w = 0; w < EVR_SUM_THREADS / 32; ++w) s += ss[w * cw + col];
-    out[v] = em == 0x7ff ? __longlong_as_double(0x7FF8000000000000LL) : sum_value(s, em);
+    out[v] = em == 0x7ff ? __longlong_as_double(0x7FF8000000000000LL) : sum_value(s, em, k2);
   }
 }
 

@@ -311,3 +311,33 @@ def test_exceptional_columns_of_terms_around_the_shared_memory(nb, nq, nrhs):
         near = [j for j in range(nrhs) if j not in far]
         assert np.array_equal(got[:, near], ref[:, near])
         assert rel_err(np.ldexp(got[:, far], -700), ref[:, far]) <= TOL
+
+
+def _remainder(n):
+    """n values of both signs, a hundred at a time of sizes down to 2^-59, that cancel but for 2^-108."""
+    rng = np.random.default_rng(n)
+    x = np.ldexp(rng.integers(1, 1 << 53, size=n).astype(np.float64), -53 - rng.integers(0, 7, size=n))
+    return np.concatenate([x, -x[rng.permutation(n)], [2.0 ** -108]]).tolist()
+
+
+@pytest.mark.parametrize("values,result", [
+    ([1.0, -1.0, 2.0 ** -110], 2.0 ** -110),
+    ([2.0 ** -115, 1.0, -1.0], 2.0 ** -115),
+    ([1.0, 2.0 ** -60, 2.0 ** -110, -1.0, -2.0 ** -60], 2.0 ** -110),
+    ([3.0, -2.0 ** -90, 5.0, -8.0, 2.0 ** -90, -2.0 ** -112] + [0.0] * 60, -2.0 ** -112),
+    ([1.0, 2.0 ** -50, -1.0], 2.0 ** -50), ([0.0, -0.0], 0.0),
+    (_remainder(255), 2.0 ** -108), (_remainder(256), 2.0 ** -108), (_remainder(2000), 2.0 ** -108)])
+@pytest.mark.parametrize("nrhs", [1, 2, 5])
+def test_sums_of_terms_that_cancel(values, result, nrhs):
+    """One function held by one term per value, on one point each: H.psi is the sum of the
+    weights times psi, here a remainder far below the terms that cancel, and above
+    2^-116 of the largest (2^-113 in lists of up to 4096), where the sums are exact."""
+    need_cuda()
+    n = len(values)
+    w = np.sign(values) + (np.asarray(values) == 0.0)
+    one = np.ones(1)
+    T = SG4Tables(1, 0, 0, [1], [1], np.zeros(1), one, one, np.zeros(1), np.zeros(1), np.zeros(n, dtype=np.int32),
+                  w, np.ones(n, dtype=np.int32), 1)
+    op = ParamOp(T, 0, V=np.abs(values))
+    psi = np.ldexp(1.0, np.arange(nrhs))[None, :]
+    assert np.array_equal(gpu_apply(op, psi), result * psi)
