@@ -1867,10 +1867,12 @@ static int hpsi_common(evr_sg4_ctx* c, int nrhs, int cshift, const double* psi, 
     CUDA_TRY(launch_list(c->geo, c->grid, smem, s, &p, 1, c->d_items, c->n_items, c->d_counter));
     launches = 1;
   } else {
-    for (long long t = 0; t < c->nb_SG; ++t) {  // one launch per Smolyak term
-      const int b0 = c->term_item_start[t], b1 = c->term_item_start[t + 1];
-      launch_multi(c->geo, b1 - b0, smem, s, &p, 1, c->d_plain_items, b1, b0, nullptr);
-      ++launches;
+    for (long long t = 0; t < c->nb_SG; ++t) {  // one launch per Smolyak term (and as many CTAs as have slabs)
+      const int b1 = c->term_item_start[t + 1];
+      for (int b = c->term_item_start[t], n; b < b1; b += n, ++launches) {
+        n = c->scratch_per_cta ? std::min(b1 - b, c->grid) : b1 - b;
+        launch_multi(c->geo, n, smem, s, &p, 1, c->d_plain_items, b + n, b, nullptr);
+      }
     }
     CUDA_TRY(cudaGetLastError());
   }

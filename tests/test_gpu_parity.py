@@ -421,3 +421,20 @@ def test_type1_coefficient_grids_in_a_multi_context_plan():
     torch.cuda.synchronize()
     for k in range(3):
         assert torch.equal(outs[k], ref[k]), k
+
+
+@pytest.mark.parametrize("nrhs,jac", [(2500, False), (700, True)])
+def test_per_term_path_with_more_items_than_slabs(nrhs, jac):
+    """One large term whose arrays lie in the CTAs' slabs of global scratch, on more
+    columns than there are slabs: the per-term path takes them in several launches."""
+    need_cuda()
+    b = SG4Basis(4, 0, A_nb=7, A_nq=8, scaleQ=np.full(4, 0.5))
+    kw = dict(Jac=np.full(b.sum_nq, 1.5)) if jac else {}
+    op = ParamOp(b, 10, V=np.random.default_rng(1).normal(size=b.sum_nq), G0=np.eye(4), G1=np.zeros((4, 4, 4)), **kw)
+    P = torch.randn((nrhs, b.N), generator=torch.Generator(device="cuda").manual_seed(2), device="cuda",
+                    dtype=torch.float64)
+    a, c = torch.empty_like(P), torch.empty_like(P)
+    op.hpsi_dev(P, a)
+    op.hpsi_dev(P, c, plain=True)
+    torch.cuda.synchronize()
+    assert torch.equal(a, c)
