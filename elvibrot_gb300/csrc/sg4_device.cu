@@ -1593,6 +1593,20 @@ extern "C" int evr_sg4_set_operator(evr_sg4_ctx* c, const evr_sg4_op_desc* op) {
 }
 
 
+// Doubles that a plan's slabs of global scratch may take in all: 16 GiB, or what
+// four CTAs an SM take with one column an item in FP64 if the operator's terms
+// need more.
+static long long slab_limit(const evr_sg4_ctx* c) {
+  return std::max((16LL << 30) / 8, 4LL * c->num_sms * nbuf_for(c) * c->z.max_nq);
+}
+
+// CTAs of a plan: no more than its items, nor than the slabs of slab doubles
+// that fit in `limit` (fixed point; the FP64 items' slabs hold one column).
+static int plan_grid(int geo, bool fx, int num_sms, size_t n_items, long long slab, long long limit) {
+  const long long grid = std::min<long long>((long long)launch_ctas(geo, fx) * num_sms, std::max<size_t>(1, n_items));
+  return (int)(fx && slab * grid > limit ? std::max(1LL, limit / slab) : grid);
+}
+
 // Work list of one H.psi over nrhs_v virtual right-hand sides: (term, rhs
 // block) items in term order with their costs, the term table with each
 // term's block size r for this nrhs_v, and the doubles of global scratch that
@@ -1615,6 +1629,7 @@ static void plan_work(const evr_sg4_ctx* c, bool fx, int nrhs_v, int smem_double
       const long long room = smem_doubles - fx_mats(c, T);
       const int want = std::min(nrhs_v, rcap);
       r = std::min(want, (int)FX_MAXR);
+      if (r > 1 && per * r > room && per * r * EVR_FX_CTAS * c->num_sms > slab_limit(c)) r = 1;
       const long long fit = std::min<long long>(nbuf, room / ((long long)T.nq * r));
       if (fit < nbuf) slab = std::max(slab, per * r);  // of which columns left to the FP64 code take all
     } else {
@@ -1655,7 +1670,8 @@ static void plan_sorted(const evr_sg4_ctx* c, int nrhs_v, std::vector<TermInfo>&
   rcap = std::min(rcap, c->rmax);
   plan_work(c, c->fx, nrhs_v, geo_smem_bytes(0, c->fx) / 8, rcap, terms, items, cost, slab);
   geo = c->geo_override >= 0 ? c->geo_override : choose_geo(c->D, items.size(), c->num_sms);
-  if (geo) plan_work(c, c->fx, nrhs_v, geo_smem_bytes(geo, c->fx) / 8, rcap, terms, items, cost, slab);
+  if (geo && !c->fx)  // (the fixed-point kernels have one shape)
+    plan_work(c, false, nrhs_v, geo_smem_bytes(geo, false) / 8, rcap, terms, items, cost, slab);
   std::vector<int> order(items.size());
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return cost[a] > cost[b]; });
@@ -1671,7 +1687,7 @@ static void plan_items(evr_sg4_ctx* c, int nrhs_v, std::vector<Item>& items, std
   plan_sorted(c, nrhs_v, c->terms, items, sorted, slab, geo);
   c->geo = geo;
   c->smem_doubles = geo_smem_bytes(geo, c->fx) / 8;
-  c->grid = launch_ctas(geo, c->fx) * c->num_sms;
+  c->grid = plan_grid(geo, c->fx, c->num_sms, items.size(), slab, slab_limit(c));
 }
 
 // a single context's device work list: every item in slot 0
@@ -2183,7 +2199,7 @@ extern "C" int evr_sg4_hpsi_noalloc(evr_sg4_ctx* c, int nrhs, const double* psi,
     off_part = off_contrib + up((size_t)c->z.sum_nb * nrhs_v * 8);
     off_slabs = off_part + up((size_t)c->N * nrhs_v * 8);
     // with large-term slabs, launch only as many CTAs as the array has slabs for
-    grid = launch_ctas(geo, c->fx) * c->num_sms;
+    grid = plan_grid(geo, c->fx, c->num_sms, sorted.size(), per_cta, slab_limit(c));
     if (per_cta > 0 && off_slabs < (size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES)
       grid = (int)std::min<long long>(grid, ((size_t)EVR_SG4_NOALLOC_SCRATCH_BYTES - off_slabs) / ((size_t)per_cta * 8));
     total = off_slabs + (size_t)per_cta * std::max(grid, 1) * 8;
@@ -2397,9 +2413,7 @@ static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int fl
   std::vector<std::vector<float>> allcost(ng);
   long long scratch_doubles = 0;
   for (MGroup& g : m->groups) {
-    const bool fx = m->fx[g.ctx_of[0]];
-    g.smem_doubles = geo_smem_bytes(g.geo, fx) / 8;
-    g.grid = launch_ctas(g.geo, fx) * sms;
+    g.smem_doubles = geo_smem_bytes(g.geo, m->fx[g.ctx_of[0]]) / 8;
   }
   for (int k = 0; k < n; ++k) {
     evr_sg4_ctx* c = ctxs[k];
@@ -2434,6 +2448,9 @@ static int multi_create(int n, evr_sg4_ctx* const* ctxs, const int* nrhs, int fl
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return allcost[gi][a] > allcost[gi][b]; });
     g.sorted.resize(all[gi].size());
     for (size_t q = 0; q < order.size(); ++q) g.sorted[q] = all[gi][order[q]];
+    long long limit = 0;
+    for (int k : g.ctx_of) limit = std::max(limit, slab_limit(ctxs[k]));
+    g.grid = plan_grid(g.geo, m->fx[g.ctx_of[0]], sms, g.sorted.size(), g.scratch_per_cta, limit);
     scratch_doubles = std::max(scratch_doubles, g.scratch_per_cta * g.grid);
     const size_t ni = std::max<size_t>(1, g.sorted.size());
     if (cudaMalloc(&g.d_items, ni * sizeof(MItem)) != cudaSuccess ||
@@ -2685,7 +2702,7 @@ int evr::bound_apply_create(evr_sg4_ctx* c, int nrhs, int transpose, const doubl
   long long per_cta = 0;
   plan_sorted(c, b->nrhs_v, terms, items, sorted, per_cta, b->geo);
   const int smem_doubles = geo_smem_bytes(b->geo, c->fx) / 8;
-  b->grid = launch_ctas(b->geo, c->fx) * c->num_sms;
+  b->grid = plan_grid(b->geo, c->fx, c->num_sms, sorted.size(), per_cta, slab_limit(c));
   auto fail = [&](const char* what) {
     cudaGetLastError();
     bound_apply_destroy(b);
