@@ -3070,7 +3070,8 @@ extern "C" int evr_sg4_diagonal(evr_sg4_ctx* c, double* diag, void* stream) {
 // per fibre, per output element, or chosen per pass).  None of them changes
 // the arithmetic of a term and right-hand side, so results are the same bits
 // for every setting.  The tuner times H.psi for each candidate on the
-// caller's block size and keeps the fastest, and records it in a JSON file
+// caller's block size (in fixed point, where only a cap of one column makes
+// another launch, that one) and keeps the fastest, and records it in a JSON file
 // keyed by the shape of the workload, so later runs apply it without timing.
 // ------------------------------------------------------------------------
 extern "C" int evr_sg4_set_plan(evr_sg4_ctx* c, int geo, int rmax, int split) {
@@ -3232,11 +3233,16 @@ extern "C" int evr_sg4_tune_plan(evr_sg4_ctx* c, int nrhs, int flags, const char
   if (!rc) {
     best.ms = best.default_ms;
     best.geo = auto_geo_of(c, nrhs, flags);
-    std::vector<int> geos = {0, 2};
+    std::vector<int> geos = {0, 2}, caps = {4, 8, 16, 32}, splits = {0, 1, 2};
     if (c->D <= EVR_NARROW_FMAX) geos.push_back(1);
+    if (c->fx) {  // one shape and one mapping, pairs of columns (the automatic plan) or single ones
+      geos = {best.geo};
+      caps = {1};
+      splits = {EVR_AUTO_SPLIT};
+    }
     for (int geo : geos)
-      for (int rmax : {4, 8, 16, 32})
-        for (int split : {0, 1, 2}) {
+      for (int rmax : caps)
+        for (int split : splits) {
           double ms = 0.0;
           if ((rc = time_plan(geo, rmax, split, &ms))) break;
           if (ms < 0.99 * best.ms) {  // a candidate must beat the best so far by more than timing noise
