@@ -147,11 +147,6 @@ class ClockSampler:
         return out
 
 
-# cycles of a warp's fixed-point multiply-add on an SM sub-partition (measured in
-# registers; an FP64 one takes 64)
-FX_CYCLES = 12.7
-
-
 def profile_traffic():
     """Per-launch DRAM traffic of the H.psi kernel from the committed ncu summary, if present."""
     p = os.path.join(ROOT, "profiles", "hpsi_items_6d_l8_20rhs.txt")
@@ -571,7 +566,7 @@ def bench_davidson12(L=4, nev=50):
 def run_ours(args, ws, rank, local):
     import torch
     import torch.distributed as dist
-    from elvibrot_gb300 import fp64_peak_tflops, lib
+    from elvibrot_gb300 import fixed_point_peak_tflops, fp64_peak_tflops, lib
     from elvibrot_gb300.configs import config, random_psi
 
     torch.cuda.set_device(local)
@@ -601,7 +596,7 @@ def run_ours(args, ws, rank, local):
     for _ in range(args.warmup):
         step()
     torch.cuda.synchronize()
-    peak = fp64_peak_tflops()
+    peak, fx_peak = fp64_peak_tflops(), fixed_point_peak_tflops()
     if ws > 1:
         dist.barrier()
     torch.cuda.synchronize()
@@ -712,9 +707,6 @@ def run_ours(args, ws, rank, local):
         cpu1_v, cpu1_steps, cpu1_dt, _ = time_oracle(model, nrhs, min_seconds=0.0, min_steps=1, max_steps=1,
                                                      seed=cfg["seed"], threads=1)
         clocks = clk.summary()
-        # the items' products run on the integer pipe (sg4_fixed.cuh)
-        sms = torch.cuda.get_device_properties(local).multi_processor_count
-        fx_peak = 2.0 * sms * 4 * 32 / FX_CYCLES * (clocks["sm_mhz"] or 2000.0) * 1e6 / 1e12
         result = {
             "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": ws, "steps": args.steps,
             "warmup": args.warmup, "ms_per_step": ms_step, "higher_is_better": True, "scaling": "weak",
@@ -726,8 +718,8 @@ def run_ours(args, ws, rank, local):
                     "d2h_bytes_per_step": 8 * N * nrhs},
             "roofline": {"bound": "int", "achieved": achieved, "peak": fx_peak, "unit": "TFLOP/s",
                          "frac": achieved / fx_peak, "traffic": profile_traffic(),
-                         "peak_source": "fixed-point multiply-adds: three mad.wide.s32, 12.7 cycles a warp and SM "
-                                        "sub-partition (measured), at the sampled SM clock",
+                         "peak_source": "in-run probe of the items' fixed-point multiply-adds (evr_probe_fixed_peak); "
+                                        "MEASURED_PEAKS.json has no integer or FP64 entry",
                          "fp64_peak": peak, "flops_per_launch": flops,
                          "hbm": {"achieved": alg_bytes / (ms_step / 1e3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                                  "frac": alg_bytes / (ms_step / 1e3) / 1e9 / hbm_peak,

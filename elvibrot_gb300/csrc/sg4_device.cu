@@ -587,6 +587,33 @@ __global__ void dfma_peak_kernel(double* out, int iters, double a, double b) {
   out[blockIdx.x * blockDim.x + threadIdx.x] = x0 + x1 + x2 + x3 + x4 + x5 + x6 + x7;
 }
 
+// The items' fixed-point multiply-add in their pattern, in registers: a fibre of
+// four values of two columns with a row of four matrix elements; the elements
+// change with every step, so that no product is formed twice.
+__global__ void fx_peak_kernel(double* out, int iters, unsigned a, unsigned b) {
+  FxAcc s[2] = {FxAcc{0, 0, 0}, FxAcc{0, 0, 0}};
+  unsigned m[8];
+  int x[16];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) m[k] = threadIdx.x * a + k * b;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) x[k] = (int)(threadIdx.x * 7919 + k * b + a);
+  for (int i = 0; i < iters; ++i) {
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      m[2 * k] += a;
+      m[2 * k + 1] ^= m[2 * k];
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        fx_mac(s[w], x[4 * k + 2 * w], x[4 * k + 2 * w + 1], make_int2((int)m[2 * k], (int)m[2 * k + 1]));
+    }
+  }
+  long long t = 0;
+#pragma unroll
+  for (int w = 0; w < 2; ++w) t += s[w].hh ^ s[w].m1 ^ s[w].m2;
+  out[blockIdx.x * blockDim.x + threadIdx.x] = (double)t;
+}
+
 // FP64 tensor-core probe: mma.sync m8n8k4 f64 (DMMA; 512 flops per warp
 // instruction) on four independent accumulator tiles per warp, in registers
 // only.  With `dfma` > 0 each step also runs that many DFMA chains per thread
@@ -2045,22 +2072,25 @@ extern "C" int evr_sg4_last_launches(const evr_sg4_ctx* c, long long* n) {
   return EVR_OK;
 }
 
-extern "C" int evr_probe_fp64_peak(double* tflops) {
+// best of three launches of a probe kernel (four blocks of 256 threads an SM),
+// which runs `ops` multiply-adds a thread
+template <class F>
+static int probe_peak(F launch, double ops, double* tflops) {
   if (!tflops) return set_error(EVR_ERR_ARG, "probe: NULL argument");
   int dev = 0, sms = 0;
   CUDA_TRY(cudaGetDevice(&dev));
   CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const int blocks = 4 * sms, threads = 256, iters = 2048;
+  const int blocks = 4 * sms, threads = 256;
   double* d = nullptr;
   CUDA_TRY(cudaMalloc(&d, sizeof(double) * blocks * threads));
   cudaEvent_t e0, e1;
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
-  dfma_peak_kernel<<<blocks, threads>>>(d, 64, 1.0000001, 1e-9);
+  launch(blocks, threads, d);
   float best = 1e30f;
   for (int rep = 0; rep < 3; ++rep) {
     cudaEventRecord(e0);
-    dfma_peak_kernel<<<blocks, threads>>>(d, iters, 1.0000001, 1e-9);
+    launch(blocks, threads, d);
     cudaEventRecord(e1);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -2072,8 +2102,20 @@ extern "C" int evr_probe_fp64_peak(double* tflops) {
   cudaEventDestroy(e1);
   cudaFree(d);
   if (e != cudaSuccess) return set_error(EVR_ERR_CUDA, "probe: %s", cudaGetErrorString(e));
-  *tflops = 2.0 * 8 * iters * (double)blocks * threads / (best * 1e-3) / 1e12;
+  *tflops = 2.0 * ops * (double)blocks * threads / (best * 1e-3) / 1e12;
   return EVR_OK;
+}
+
+extern "C" int evr_probe_fp64_peak(double* tflops) {
+  const int iters = 2048;
+  return probe_peak([=](int b, int t, double* d) { dfma_peak_kernel<<<b, t>>>(d, iters, 1.0000001, 1e-9); }, 8.0 * iters,
+                    tflops);
+}
+
+extern "C" int evr_probe_fixed_peak(double* tflops) {
+  const int iters = 4096;
+  return probe_peak([=](int b, int t, double* d) { fx_peak_kernel<<<b, t>>>(d, iters, 12345, 54321); }, 8.0 * iters,
+                    tflops);
 }
 
 extern "C" int evr_probe_fp64_pipes(double* dfma_tflops, double* dmma_tflops, double* mixed_tflops) {

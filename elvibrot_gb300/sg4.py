@@ -121,6 +121,7 @@ def _declare(L):
         "evr_sg4_last_launches": [vp, ctypes.POINTER(ll)],
         "evr_sg4_last_geometry": [vp, ctypes.POINTER(ctypes.c_int), ctypes.POINTER(ctypes.c_int)],
         "evr_probe_fp64_peak": [dp],
+        "evr_probe_fixed_peak": [dp],
         "evr_probe_fp64_pipes": [dp, dp, dp],
         "evr_sg4_set_plan": [vp, ctypes.c_int, ctypes.c_int, ctypes.c_int],
         "evr_sg4_get_plan": [vp, ip, ip, ip],
@@ -663,6 +664,13 @@ def hpsi_multi(ops, psis, outs, E0=None, Esc=None, transpose: bool = False, stre
 def fp64_peak_tflops() -> float:
     t = ctypes.c_double()
     check(lib().evr_probe_fp64_peak(ctypes.byref(t)))
+    return t.value
+
+
+def fixed_point_peak_tflops() -> float:
+    """The items' fixed-point multiply-adds, two operations each, in TFLOP/s."""
+    t = ctypes.c_double()
+    check(lib().evr_probe_fixed_peak(ctypes.byref(t)))
     return t.value
 
 

@@ -478,6 +478,9 @@ const char* evr_sg4_last_error(void);
 /* Measured FP64 FMA throughput of the current device in TFLOP/s (a short
  * in-bounds DFMA loop; used as the roofline denominator). */
 int evr_probe_fp64_peak(double* tflops);
+/* The same for the fixed-point multiply-adds of the H.psi items (60-bit values in
+ * two limbs, three 32 x 32 + 64-bit products each), two operations each. */
+int evr_probe_fixed_peak(double* tflops);
 
 /* The FP64 pipes of the current device, each in TFLOP/s: the DFMA loop
  * above, FP64 tensor-core MMA alone (mma.sync m8n8k4 f64, registers only),
