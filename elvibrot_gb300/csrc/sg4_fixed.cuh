@@ -1,12 +1,12 @@
 // sg4_fixed.cuh -- the H.psi work items in block fixed point.
 //
-// GB300 runs two FP64 operations a clock and SM, but 61 32 x 32 + 64-bit
-// integer multiply-adds (mad.wide.s32; both measured with an instruction
-// probe), so the items' contractions -- the 1-D passes, the derivatives, the
-// metric -- run on the integer pipe: a value is a 60-bit integer in two limbs,
+// GB300 runs two FP64 multiply-adds a clock and SM, but nine to ten of these in
+// fixed point (evr_probe_fp64_peak: 1.25 TFLOP/s, evr_probe_fixed_peak: 5.8), so
+// the items' contractions -- the 1-D passes, the derivatives, the metric -- run
+// on the integer pipe: a value is a 60-bit integer in two limbs,
 //   value = (h 2^29 + l) 2^e,  |l| <= 2^28,  |h| <= 2^30,
 // with one exponent e per right-hand side of an item and stage, and a
-// multiply-add is three mad.wide.s32 into two 64-bit accumulators,
+// multiply-add is three 32 x 32 + 64-bit ones into two 64-bit accumulators,
 //   hh += xh mh,  mid += xh ml + xl mh
 // (the xl ml product is below 2^-60 of full scale).  Matrices are scaled so
 // that the absolute sum of every row is at most 2^58, so a pass cannot
@@ -14,7 +14,8 @@
 // side, and the next pass shifts the headroom it finds there into its result,
 // so each pass loses only the bits by which its own row-sum bound exceeds its
 // result (two to four), not the product of all of them.  That keeps 55 to 57
-// bits of each stage's largest value, against the 53 of a double.
+// bits of each stage's largest value, at every point alike; a double has 53 of
+// each value.
 //
 // A right-hand side whose largest entry in a term lies outside 2^+-300 (all
 // subnormal, for instance), or is not finite, and one whose result is small
@@ -856,9 +857,10 @@ __device__ __forceinline__ void run_item_fx(const KParams& p, ItemShared& it, Fx
     else fx_body<2, false>(p, it, fs, FxBufs<2, false>{X, Tb, slab, nfit, NQR});
   }
   if (fs.bad) {
-    const int bad = fs.bad;
-    const bool in = (long long)narr * NQR <= p.smem_doubles;  // else the plan has a slab for this item's arrays
-    fx_item_fp64(p, it, in ? reinterpret_cast<double*>(fx_sm) : reinterpret_cast<double*>(slab), rhs0, bad, fs.tile);
+    // the arrays of the item's columns, in the plan's slab where they exceed shared memory
+    const bool in = (p.type == 10 ? D + 1LL : 2LL) * it.nq_t * r <= p.smem_doubles;
+    double* A = in ? reinterpret_cast<double*>(fx_sm) : p.gscratch + (long long)blockIdx.x * p.scratch_per_cta;
+    fx_item_fp64(p, it, A, rhs0, fs.bad, fs.tile);
   }
 }
 
