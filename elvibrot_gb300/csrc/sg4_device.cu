@@ -2915,7 +2915,7 @@ evr::FieldPairView evr::field_pair_view(const FieldPair* f) {
 // inner one: a grid->basis transform of the field f with the "pattern"
 // matrices P_l in place of RBGwrho.  Per term: one transform per pattern
 // (V; D^2 G_ij terms for type 10, -1/2 each; F2/F1 terms for type 1), the
-// weighted result into the contribution buffer, then the ordered
+// weighted result into the contribution buffer, then the
 // accumulation of evr_sg4_hpsi.  A few H.psi-equivalents of work instead of
 // N/64 H.psi calls on blocks of unit vectors.  Type 10 with Jac or rho (the
 // -1/2/(Jac s) factor does not factor per mode), several channels and

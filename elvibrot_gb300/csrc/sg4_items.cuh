@@ -46,9 +46,10 @@ namespace evr {
 #endif
 #define EVR_MID_FMAX 12
 // The fixed-point kernels have one shape for every geometry: seven CTAs of 128
-// threads an SM (72 registers, 29.5 KB).  The item's phases end in barriers,
+// threads an SM (72 registers, 29.5 KB; a 480-byte stack frame, 180 bytes of
+// spill stores and 360 of loads).  The item's phases end in barriers,
 // which other CTAs fill.  Measured on the 6-D benchmark (20 vectors, two columns
-// an item): seven CTAs of 128 threads 2.82 ms, six 2.89, eight (64 registers,
+// an item) when chosen: seven CTAs of 128 threads 2.82 ms, six 2.89, eight (64 registers,
 // spills) 3.52; in an earlier build, against six at 3.20: five of 192 3.65, four
 // of 192 3.36, four of 256 3.65, three of 256 3.73, two of 512 4.45, two of 384
 // 4.34, four of 128 with four columns an item 3.49, two of 256 with four 3.88.

@@ -1453,7 +1453,7 @@ extern "C" int evr_sg4_multi_cheby_propagate(evr_sg4_multi* m, const evr_cheby_o
   // unchanged since the recording, one whole step -- the start of every
   // context's recurrence, each order's merged H.psi (bound parameter blocks:
   // the source vector alternates between two buffers, so two blocks) with the
-  // contexts' ordered accumulations and recurrence updates, and the norms of
+  // contexts' accumulations and recurrence updates, and the norms of
   // the last terms into pinned memory -- replays as one CUDA graph.  A context
   // whose step diverges is then redone eagerly, alone with the other diverged
   // ones; the same kernels run either way, so the bits are those of the eager

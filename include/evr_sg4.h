@@ -340,7 +340,7 @@ int evr_sg4_davidson(evr_sg4_ctx* c, const evr_davidson_opts* o, const double* g
  * sub_NewVec_Davidson, sub_module_Davidson.f90:1306).  Computed term by
  * term: each Smolyak term's diagonal is a grid->basis transform of its
  * fields with per-mode matrices (RBGwrho.D o (D.RGB)^T), one transform per
- * field term, then the weighted, term-ordered accumulation of H.psi.  Type 10
+ * field term, then the weighted accumulation of H.psi.  Type 10
  * with Jac or rho grids, type 1 with coefficient grids, several channels and
  * streamed fields use evr_sg4_diagonal_by_apply. */
 int evr_sg4_diagonal(evr_sg4_ctx* c, double* diag, void* stream);
@@ -372,7 +372,7 @@ int evr_sg4_cheby_propagate(evr_sg4_ctx* c, const evr_cheby_opts* o, int nrhs, d
 /* Several independent Hamiltonians (contexts of any D, L and operator type)
  * applied in ONE persistent launch: the (context, term, rhs block) items of
  * all of them are merged into one cost-sorted work list, followed by each
- * context's ordered accumulation (1 + 2n launches).  No counterpart in the
+ * context's accumulation (1 + 2n launches).  No counterpart in the
  * reference, which applies one para_Op per sub_TabOpPsi call
  * (SRC/sub_Operator/sub_OpPsi.f90:705); this batches its independent
  * Hamiltonians (the uneven-instance workload) on one GPU.
@@ -414,7 +414,7 @@ int evr_sg4_multi_destroy(evr_sg4_multi* m);
  * interleaved complex128 N_k x nrhs_k, propagated in place; autocorr[k]: host
  * complex [(nsteps+1) x nrhs_k] = <psi_k(0) | psi_k(t_j)>, or NULL.  Unless
  * o[0].no_graph, a step with every context in it (each order's merged launch,
- * the ordered accumulations and recurrence updates of every context) is
+ * the accumulations and recurrence updates of every context) is
  * recorded once as a CUDA graph and replayed while the bounds stay the same;
  * diverged contexts are redone eagerly (the same kernels, the same bits). */
 int evr_sg4_multi_cheby_propagate(evr_sg4_multi* m, const evr_cheby_opts* o, double* const* psi,
