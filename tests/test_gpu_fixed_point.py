@@ -341,3 +341,29 @@ def test_sums_of_terms_that_cancel(values, result, nrhs):
     op = ParamOp(T, 0, V=np.abs(values))
     psi = np.ldexp(1.0, np.arange(nrhs))[None, :]
     assert np.array_equal(gpu_apply(op, psi), result * psi)
+
+
+def test_slabs_of_large_terms_stay_within_their_limit():
+    """One term of 8^6 points, type 10: two columns of 7 arrays take 29 MB a CTA, 31 GB on
+    seven CTAs an SM.  The plan takes single columns, and no more CTAs than items; every
+    column has the bits of a call on a few."""
+    need_cuda()
+    b = SG4Basis(6, 0, A_nb=2, A_nq=8, scaleQ=np.full(6, 0.5))
+    V = np.random.default_rng(6).normal(size=b.sum_nq)
+    op = ParamOp(b, 10, V=V, G0=np.eye(6), G1=np.zeros((6, 6, 6)))
+    P = torch.randn((1300, b.N), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda",
+                    dtype=torch.float64)
+    few, out = torch.empty_like(P[:3]), torch.empty_like(P)
+    free = [torch.cuda.mem_get_info()[0]]
+    for x, y in ((P[:3].contiguous(), few), (P, out)):
+        op.hpsi_dev(x, y)
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    array = 8 * 7 * 8 ** 6
+    assert free[0] - free[1] <= 6 * array + (64 << 20)      # three items
+    assert free[0] - free[2] <= (16 << 30) + (64 << 20)
+    assert torch.equal(out[:3], few)
+    x = np.ascontiguousarray(P[:3].cpu().numpy().T)
+    G = np.concatenate([np.repeat(np.eye(6).ravel(), b.sum_nq)])
+    O = OracleSG4(6, 0, 0, 2, 0, 8, 0, scaleQ=np.full(6, 0.5))
+    assert rel_err(few.cpu().numpy().T, O.hpsi(x, type_op=10, V=V, G=G)) <= TOL
